@@ -73,13 +73,13 @@ def draw(rng):
     dtype = rng.choice(["bf16", "bf16", "fp16"])
     if kind == "decode_step":
         batch = _log(rng, 1, 64)
-        hi = max(_log(rng, 64, 8192) // 1, 64)
+        hi = _log(rng, 64, 8192)
         return {"kind": kind, "batch": batch, "lo": max(hi // 10, 1), "hi": hi, "page": rng.choice([16, 64]),
                 "hq": hq, "hkv": hkv, "dim": rng.choice([64, 128]), "dtype": dtype,
                 "window": rng.choice([0, 0, 0, 1024])}
     if kind == "decode":
-        batch = _log(rng, 1, 64)
         hi = _log(rng, 256, 32768)
+        batch = min(_log(rng, 1, 64), (1 << 20) // hi)
         return {"kind": kind, "batch": batch, "lo": max(hi // rng.choice([2, 30]), 1), "hi": hi,
                 "page": rng.choice([16, 64]), "hq": 32, "hkv": 8, "dim": rng.choice([64, 96, 128, 128]),
                 "dtype": dtype, "window": rng.choice([0, 0, 0, 4096]), "softcap": rng.choice([0.0, 0.0, 0.0, 30.0])}
@@ -88,11 +88,12 @@ def draw(rng):
         return {"kind": kind, "batch": _log(rng, 1, 32), "lo": max(hi // 30, 1), "hi": hi, "hq": 32, "hkv": 8,
                 "dim": rng.choice([64, 128, 128]), "dtype": dtype}
     if kind == "prefill":
-        hi = _log(rng, 16, 8192)
+        causal = rng.random() < 0.85
+        hi = _log(rng, 16, 8192 if causal else 4096)
         batch = max(1, min(_log(rng, 1, 16), 32768 // hi))
         return {"kind": kind, "batch": batch, "lo": max(hi // rng.choice([1, 4, 40]), 1), "hi": hi,
                 "hq": min(hq, 32), "hkv": hkv, "dim": rng.choice([64, 80, 96, 128, 128, 128]), "dtype": dtype,
-                "causal": rng.random() < 0.85}
+                "causal": causal}
     if kind == "chunked":
         hi = _log(rng, 16, 2048)
         return {"kind": kind, "batch": _log(rng, 1, 8), "lo": max(hi // 3, 1), "hi": hi, "past": rng.choice([0, 1]) *
