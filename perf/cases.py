@@ -110,8 +110,10 @@ def draw(rng):
         return {"kind": kind, "tokens": _log(rng, 16, 32768), "experts": experts, "groups": groups, "keep": keep,
                 "topk": topk}
     if kind == "gate":
-        return {"kind": kind, "tokens": _log(rng, 256, 16384), "experts": rng.choice([8, 16, 64, 128]),
-                "topk": rng.choice([1, 2, 4, 8]), "factor": rng.choice([1.0, 1.25, 2.0]),
+        experts, topk = rng.choice([8, 16, 64, 128]), rng.choice([1, 2, 4, 8])
+        # a capacity above the number of tokens has no list to fill it with
+        factor = rng.choice([f for f in (1.0, 1.25, 2.0) if f * topk <= experts])
+        return {"kind": kind, "tokens": _log(rng, 256, 16384), "experts": experts, "topk": topk, "factor": factor,
                 "full_grad": rng.random() < 0.6, "dtype": "fp32"}
     return {"kind": "silu", "tokens": _log(rng, 1, 8192), "inter": rng.choice([_log(rng, 500, 14336), 4096, 11008]),
             "dtype": rng.choice(["bf16", "bf16", "fp16", "fp32"])}
