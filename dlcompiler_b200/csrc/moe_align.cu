@@ -11,92 +11,60 @@
 //   * num_tokens_post_padded[0] is the padded length,
 //   * block_start[e] (E + 1 entries) is the first block of expert e.
 // Slots whose id is outside [0, E) (experts owned by another rank) are dropped.
-// All outputs are integer and bit-exact reproducible: positions are derived
-// from prefix sums and warp match masks, never from atomics on positions.
+// All outputs are integer and bit-exact reproducible (the sort itself: slot_sort.cuh).
 #include "common.cuh"
+#include "slot_sort.cuh"
 
 namespace dlb {
 
 constexpr int ALIGN_THREADS = 1024;
-constexpr int ALIGN_WARPS = ALIGN_THREADS / 32;
 
+// Bounded by latency, not by bytes (64 KB in, 64 KB out at 16000 slots): the chain is one id load, the count,
+// a cluster barrier, the scan over experts and one more walk.
 template <typename IdT>
-__global__ void __launch_bounds__(ALIGN_THREADS) moe_align_kernel(
+__global__ void __launch_bounds__(SORT_THREADS) moe_align_kernel(
     const IdT* __restrict__ topk_ids, int32_t* __restrict__ sorted_token_ids, int32_t* __restrict__ expert_ids,
     int32_t* __restrict__ num_tokens_post_padded, int32_t* __restrict__ block_start, int numel, int num_experts,
     int block, int sorted_capacity, int expert_ids_capacity) {
   extern __shared__ int32_t smem[];
-  int32_t* counts = smem;                          // [E]    tokens per expert
-  int32_t* seg_off = counts + num_experts;         // [E+1]  padded start of each expert
-  int32_t* running = seg_off + num_experts + 1;    // [E]    tokens already placed per expert
-  int32_t* warp_cnt = running + num_experts;       // [ALIGN_WARPS][E]
-  const int tid = threadIdx.x;
-  const int lane = tid & 31;
-  const int warp = tid >> 5;
-
-  for (int e = tid; e < num_experts; e += ALIGN_THREADS) {
-    counts[e] = 0;
-    running[e] = 0;
+  SlotSort sort(smem, num_experts, numel);
+  auto id_at = [&](int slot) {
+    const int64_t v = (int64_t)topk_ids[slot];
+    return v >= 0 && v < num_experts ? (int)v : -1;
+  };
+  sort.count_slots(id_at);
+  sort.block_scan([&](int e) { return (sort.count[e] + block - 1) / block; });   // start[e] = first block of e
+  const int* first = sort.start;
+  const int blocks = first[num_experts];
+  sort.place(id_at, [&](int slot, int e, int at) {
+    const int pos = first[e] * block + at;
+    if (pos < sorted_capacity) sorted_token_ids[pos] = slot;
+  });
+  // what no slot fills: each expert's padding, the list behind the last block, and the block owners
+  const int tid = sort.rank * SORT_THREADS + threadIdx.x, threads = sort.ctas * SORT_THREADS;
+  if (block > 1) {
+    const int lane = threadIdx.x & 31;
+    for (int e = tid >> 5; e < num_experts; e += threads >> 5)
+      for (int i = first[e] * block + sort.count[e] + lane; i < min(first[e + 1] * block, sorted_capacity); i += 32)
+        sorted_token_ids[i] = numel;
   }
-  __syncthreads();
-  // 1. histogram (integer adds commute, so shared atomics stay deterministic)
-  for (int i = tid; i < numel; i += ALIGN_THREADS) {
-    const int64_t e = (int64_t)topk_ids[i];
-    if (e >= 0 && e < num_experts) atomicAdd(&counts[(int)e], 1);
-  }
-  __syncthreads();
-  // 2. exclusive scan of the padded counts (serial over experts: E <= 1024)
-  if (tid == 0) {
-    int acc = 0;
-    int blk = 0;
-    for (int e = 0; e < num_experts; ++e) {
-      seg_off[e] = acc;
-      block_start[e] = blk;
-      const int nb = (counts[e] + block - 1) / block;
-      for (int b = 0; b < nb; ++b)
-        if (blk + b < expert_ids_capacity) expert_ids[blk + b] = e;
-      blk += nb;
-      acc += nb * block;
-    }
-    seg_off[num_experts] = acc;
-    block_start[num_experts] = blk;
-    num_tokens_post_padded[0] = acc;
-    for (int b = blk; b < expert_ids_capacity; ++b) expert_ids[b] = -1;
-  }
-  // 3. sentinel fill of the whole capacity
-  for (int i = tid; i < sorted_capacity; i += ALIGN_THREADS) sorted_token_ids[i] = numel;
-  __syncthreads();
-  // 4. stable placement, ALIGN_THREADS consecutive slots per round
-  for (int base = 0; base < numel; base += ALIGN_THREADS) {
-    for (int i = tid; i < ALIGN_WARPS * num_experts; i += ALIGN_THREADS) warp_cnt[i] = 0;
-    __syncthreads();
-    const int slot = base + tid;
-    int e = -1;
-    if (slot < numel) {
-      const int64_t v = (int64_t)topk_ids[slot];
-      if (v >= 0 && v < num_experts) e = (int)v;
-    }
-    const unsigned peers = __match_any_sync(0xffffffffu, e);
-    const int rank_in_warp = __popc(peers & ((1u << lane) - 1u));
-    if (e >= 0 && rank_in_warp == 0) warp_cnt[warp * num_experts + e] = __popc(peers);
-    __syncthreads();
-    // exclusive scan over warps, one thread per expert
-    for (int x = tid; x < num_experts; x += ALIGN_THREADS) {
-      int acc = running[x];
-      for (int w = 0; w < ALIGN_WARPS; ++w) {
-        const int c = warp_cnt[w * num_experts + x];
-        warp_cnt[w * num_experts + x] = acc;
-        acc += c;
+  for (int i = blocks * block + tid; i < sorted_capacity; i += threads) sorted_token_ids[i] = numel;
+  if (expert_ids != nullptr) {
+    for (int b = tid; b < expert_ids_capacity; b += threads) {
+      int lo = 0, hi = num_experts;      // last expert whose first block is <= b (empty ones share it with the next)
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (first[mid] <= b) lo = mid;
+        else hi = mid;
       }
-      running[x] = acc;
+      expert_ids[b] = b < blocks ? lo : -1;
     }
-    __syncthreads();
-    if (e >= 0) {
-      const int pos = seg_off[e] + warp_cnt[warp * num_experts + e] + rank_in_warp;
-      if (pos < sorted_capacity) sorted_token_ids[pos] = slot;
-    }
-    __syncthreads();
   }
+  if (sort.rank == 0) {
+    for (int e = threadIdx.x; e <= num_experts; e += SORT_THREADS) block_start[e] = first[e];
+    if (threadIdx.x == 0) num_tokens_post_padded[0] = blocks * block;
+  }
+  sort.finish();
 }
 
 // dst[p, :] = src[sorted_token_ids[p] / top_k, :]  (zeros for sentinel rows).
@@ -236,7 +204,7 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   DLB_CHECK_ARG(num_experts >= 1 && num_experts <= 1024, DLB_ERR_UNSUPPORTED, "moe_align: experts=%d not in [1,1024]",
                 num_experts);
   DLB_CHECK_ARG(block >= 1, DLB_ERR_BAD_ARG, "moe_align: block=%d", block);
-  DLB_CHECK_ARG(sorted_token_ids && expert_ids && num_tokens_post_padded && block_start, DLB_ERR_BAD_ARG,
+  DLB_CHECK_ARG(sorted_token_ids && num_tokens_post_padded && block_start, DLB_ERR_BAD_ARG,
                 "moe_align: null output pointer");
   DLB_CHECK_ARG(numel == 0 || topk_ids != nullptr, DLB_ERR_BAD_ARG, "moe_align: null topk_ids");
   // worst case padded length: every expert wastes block-1 entries
@@ -244,23 +212,23 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   const int64_t need = numel == 0 ? 0 : (worst < (numel + block - 1) / block * block ? worst : worst);
   DLB_CHECK_ARG(sorted_capacity >= need && sorted_capacity < (1LL << 31), DLB_ERR_BAD_ARG,
                 "moe_align: sorted_token_ids capacity %lld < %lld", (long long)sorted_capacity, (long long)need);
-  DLB_CHECK_ARG(expert_ids_capacity >= (need + block - 1) / block, DLB_ERR_BAD_ARG,
+  DLB_CHECK_ARG(expert_ids == nullptr || expert_ids_capacity >= (need + block - 1) / block, DLB_ERR_BAD_ARG,
                 "moe_align: expert_ids capacity %lld too small", (long long)expert_ids_capacity);
-  const size_t smem = sizeof(int32_t) * ((size_t)num_experts * (3 + ALIGN_WARPS) + 1);
+  const size_t smem = sizeof(int32_t) * sort_smem_ints(num_experts);
+  const int ctas = sort_cluster_size(numel);
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e;
-  if (ids_are_int64) {
-    e = cudaFuncSetAttribute(moe_align_kernel<int64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { set_last_error("moe_align: smem attribute: %s", cudaGetErrorString(e)); return (int)e; }
-    moe_align_kernel<int64_t><<<1, ALIGN_THREADS, smem, s>>>(
-        (const int64_t*)topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, block_start, (int)numel,
-        num_experts, block, (int)sorted_capacity, (int)expert_ids_capacity);
-  } else {
-    e = cudaFuncSetAttribute(moe_align_kernel<int32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) { set_last_error("moe_align: smem attribute: %s", cudaGetErrorString(e)); return (int)e; }
-    moe_align_kernel<int32_t><<<1, ALIGN_THREADS, smem, s>>>(
-        (const int32_t*)topk_ids, sorted_token_ids, expert_ids, num_tokens_post_padded, block_start, (int)numel,
-        num_experts, block, (int)sorted_capacity, (int)expert_ids_capacity);
+  if (ids_are_int64)
+    e = launch_one_cluster(moe_align_kernel<int64_t>, ctas, smem, s, (const int64_t*)topk_ids, sorted_token_ids,
+                           expert_ids, num_tokens_post_padded, block_start, (int)numel, num_experts, block,
+                           (int)sorted_capacity, (int)expert_ids_capacity);
+  else
+    e = launch_one_cluster(moe_align_kernel<int32_t>, ctas, smem, s, (const int32_t*)topk_ids, sorted_token_ids,
+                           expert_ids, num_tokens_post_padded, block_start, (int)numel, num_experts, block,
+                           (int)sorted_capacity, (int)expert_ids_capacity);
+  if (e != cudaSuccess) {
+    set_last_error("moe_align: launch: %s", cudaGetErrorString(e));
+    return (int)e;
   }
   DLB_CUDA_LAUNCH_CHECK();
   return DLB_OK;

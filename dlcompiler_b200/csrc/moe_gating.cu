@@ -20,6 +20,7 @@
 #include <math_constants.h>
 
 #include "common.cuh"
+#include "slot_sort.cuh"
 
 namespace dlb {
 
@@ -43,6 +44,7 @@ struct GatingParams {
   float scale;
   int lanes_per_group = 1;        // filled by launch_gating
   int lanes_per_group_log2 = 0;
+  float* colsum = nullptr;        // GATE form: [CTAs, E] sums of the CTA's probability rows
 };
 
 // sigmoid evaluated by a FIXED sequence of correctly-rounded fp32 operations (fused
@@ -227,9 +229,10 @@ __device__ __forceinline__ void topk_rounds(uint32_t head, const uint32_t* __res
 // and 16-byte aligned rows and bias, so no bounds checks and only vector loads.  LG >= 0 fixes the lanes per
 // group at 2^LG with all 32 lanes in groups, and TOPK > 0 fixes top_k, so that the shuffle trees, the group
 // ranking and the rounds unroll (the DeepSeek-V3 shape: 256 experts, 8 groups, top-8); LG = -1 / TOPK = 0
-// read them from the parameters.
+// read them from the parameters.  GATE: the capacity-limited gate's form: the probabilities are stored, their
+// column sums over the CTA's tokens too, the ids choice-major ([K, T]), and no weights.
 constexpr int kGateMinBlocks = 6;   // 40 registers per thread, six CTAs per SM (1 % faster than 48 registers / five)
-template <int VPL, bool FULL, int LG = -1, int TOPK = 0>
+template <int VPL, bool FULL, int LG = -1, int TOPK = 0, bool GATE = false>
 __global__ void __launch_bounds__(GateShape<VPL>::WARPS * 32, LG >= 0 ? kGateMinBlocks : 1)
 grouped_topk_kernel(GatingParams p) {
   constexpr int WARPS = GateShape<VPL>::WARPS, LIST = GateShape<VPL>::LIST;
@@ -239,11 +242,12 @@ grouped_topk_kernel(GatingParams p) {
   __shared__ __align__(16) float sm_s[WARPS][32 * VPL];          // per warp: every expert's un-biased score
   __shared__ __align__(16) uint32_t sm_list[WARPS][32 * LIST];   // per warp: each lane's keys sorted descending, then 0
   __shared__ __align__(8) uint2 sm_win[WARPS][32];               // per warp: round k's winner (key, lane | run << 8)
-  if (token >= p.tokens) return;  // whole warp leaves together
+  const bool live = token < p.tokens;
+  if (!GATE && !live) return;     // whole warp leaves together; with GATE it takes part in the column sums' barrier
 
   const int E = p.experts;
   const int e0 = lane * VPL;
-  const float* row = p.logits + token * p.ld;
+  const float* row = p.logits + (live ? token : 0) * p.ld;
   auto valid = [&](int v) { return FULL || e0 + v < E; };
 
   float s[VPL];  // un-biased score (sigmoid or softmax probability)
@@ -302,7 +306,7 @@ grouped_topk_kernel(GatingParams p) {
 #pragma unroll
     for (int v = 0; v < VPL; ++v) s[v] = valid(v) ? s[v] / sum : -CUDART_INF_F;
   }
-  if (p.probs != nullptr) {
+  if (p.probs != nullptr && live) {
 #pragma unroll
     for (int v = 0; v < VPL; ++v)
       if (valid(v)) p.probs[token * E + e0 + v] = s[v];
@@ -359,6 +363,15 @@ grouped_topk_kernel(GatingParams p) {
     for (int v = 0; v < VPL; ++v) {
       wkeys[e0 + v] = okey[v];
       wscores[e0 + v] = s[v];
+    }
+  }
+  if constexpr (GATE) {
+    __syncthreads();
+    const int warps = (int)min((int64_t)WARPS, p.tokens - (int64_t)blockIdx.x * WARPS);
+    for (int e = threadIdx.x; e < E; e += WARPS * 32) {
+      float acc = 0.f;
+      for (int w = 0; w < warps; ++w) acc += sm_s[w][e];
+      p.colsum[(int64_t)blockIdx.x * E + e] = acc;
     }
   }
   uint32_t* my_list = sm_list[threadIdx.x >> 5] + lane * LIST;
@@ -449,6 +462,10 @@ grouped_topk_kernel(GatingParams p) {
     }
   }
   const int my_id = my_owner * VPL + my_v;
+  if constexpr (GATE) {
+    if (live && lane < top_k) p.ids[(int64_t)lane * p.tokens + token] = my_id;
+    return;
+  }
   const float my_w = (lane < top_k) ? wscores[my_id] : 0.f;
   float wsum = my_w;
   // lanes >= top_k hold 0, so with top_k <= 8 the first two levels of the tree add exact zeros and are skipped
@@ -524,96 +541,137 @@ __global__ void __launch_bounds__(256) gshard_colsum_stage1(const float* __restr
     part[(int64_t)blockIdx.x * E + e] = acc;
   }
 }
-// me[e] = sum / S;  ce[e] = first-choice count / S;  l_aux = mean(me * ce) * E * E
-__global__ void __launch_bounds__(256) gshard_aux_kernel(const float* __restrict__ part, int nblk,
-                                                         const int32_t* __restrict__ ids_km /* [K*S] */,
-                                                         int64_t S, int E, float* __restrict__ me,
-                                                         float* __restrict__ ce, float* __restrict__ l_aux) {
-  extern __shared__ float sh[];   // [E] first-choice counts, then reduction scratch
-  float* cnt = sh;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) cnt[e] = 0.f;
+// Everything behind the gate's choices in one launch of one cluster: queue positions (a stable sort of the
+// choice-major slots by expert), the per-expert token lists, the column means and the auxiliary loss
+//   me[e] = mean over tokens of gates[:, e];  ce[e] = first-choice count / S;  l_aux = mean(me * ce) * E * E,
+// the routing weights (choices beyond the capacity dropped, the kept gate values normalised) and the filling of
+// the lists' unused slots.  `part` holds `rows` partial column sums; they are added in a fixed order.
+// Latency-bound: 4096 tokens x 8 choices over 64 experts move about 3 MB.  As six launches (the sort, the sums,
+// the queue, the fill and the weights one by one) it took 303 us on B200, 274 of them in the one-CTA sort; as one
+// launch it takes 22 us.
+__global__ void __launch_bounds__(SORT_THREADS) gshard_assign_kernel(
+    const float* __restrict__ gates, const int32_t* __restrict__ ids_km /* [K*S] */, const float* __restrict__ part,
+    int rows, int32_t* loc, float* __restrict__ me, float* __restrict__ ce, float* __restrict__ l_aux,
+    int32_t* __restrict__ ec_idx, float* __restrict__ weights, int64_t* select, int S, int E, int K, int capacity,
+    float eps) {
+  extern __shared__ int32_t smem[];
+  SlotSort sort(smem, E, K * S);
+  int* first = smem + (SORT_WARPS * sort_pitch(E) + 4 * E + 1 + 2 * SORT_WARPS);   // [E] first choices in this CTA's segments
+  float* colsum = reinterpret_cast<float*>(first + E);                              // [E] this CTA's share of the sums
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  auto cl = cooperative_groups::this_cluster();
+  for (int e = threadIdx.x; e < E; e += SORT_THREADS) first[e] = 0;
   __syncthreads();
-  for (int64_t i = threadIdx.x; i < S; i += blockDim.x) atomicAdd(&cnt[ids_km[i]], 1.0f);   // integers: exact
+  for (int s = sort.lo + lane; s < min(sort.hi, S); s += 32) atomicAdd(&first[ids_km[s]], 1);   // the first S slots
+  auto id_at = [&](int slot) {
+    const int v = ids_km[slot];
+    return v >= 0 && v < E ? v : -1;
+  };
+  sort.count_slots(id_at);
+  sort.place(id_at, [&](int slot, int e, int at) {
+    loc[slot] = at;
+    if (at < capacity) select[(int64_t)e * capacity + at] = slot % S;   // token of the at-th kept choice
+  });
   __syncthreads();
-  float local = 0.f;
-  for (int e = threadIdx.x; e < E; e += blockDim.x) {
-    float acc = 0.f;
-    for (int b = 0; b < nblk; ++b) acc += part[(int64_t)b * E + e];
-    const float m = acc / (float)S, c = cnt[e] / (float)S;
-    me[e] = m;
-    ce[e] = c;
-    local += m * c;
+  {
+    // column sums: a warp per row of this CTA's share, then the warps one after the other
+    float* red = reinterpret_cast<float*>(sort.table);
+    const int per = (rows + sort.ctas - 1) / sort.ctas, r0 = sort.rank * per, r1 = min(rows, r0 + per);
+    for (int e = lane; e < E; e += 32) {
+      float acc = 0.f;
+      for (int r = r0 + warp; r < r1; r += SORT_WARPS) acc += part[(int64_t)r * E + e];
+      red[warp * sort.pitch + e] = acc;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < E; e += SORT_THREADS) {
+      float acc = 0.f;
+      for (int w = 0; w < SORT_WARPS; ++w) acc += red[w * sort.pitch + e];
+      colsum[e] = acc;
+    }
   }
-  __shared__ float red[8];
+  sort.finish();
+  __syncthreads();
+  cl.sync();          // loc, the lists, the sums and the counts of every CTA are in place
+  if (sort.rank == 0) {
+    float local = 0.f;
+    for (int e = threadIdx.x; e < E; e += SORT_THREADS) {
+      float acc = 0.f;
+      int cnt = 0;
+      for (int r = 0; r < sort.ctas; ++r) {
+        acc += *cl.map_shared_rank(&colsum[e], r);
+        cnt += *cl.map_shared_rank(&first[e], r);
+      }
+      const float m = acc / (float)S, c = (float)cnt / (float)S;
+      me[e] = m;
+      ce[e] = c;
+      local += m * c;
+    }
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = local;
+    for (int o = 16; o > 0; o >>= 1) local += __shfl_xor_sync(0xffffffffu, local, o);
+    float* red = reinterpret_cast<float*>(sort.scratch);
+    if (lane == 0) red[warp] = local;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      float t = 0.f;
+      for (int w = 0; w < SORT_WARPS; ++w) t += red[w];
+      l_aux[0] = t / (float)E * (float)E * (float)E;
+    }
+  }
+  // per token: drop choices beyond capacity, normalise the kept gate values, emit e * capacity + position
+  for (int s = sort.rank * SORT_THREADS + threadIdx.x; s < S; s += sort.ctas * SORT_THREADS) {
+    float denom = 0.f;
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      const float g = gates[(int64_t)s * E + ids_km[k * S + s]];
+      if (__ldcg(loc + k * S + s) < capacity) denom += g;
+    }
+    denom = fmaxf(denom, eps);
+#pragma unroll 4
+    for (int k = 0; k < K; ++k) {
+      const int e = ids_km[k * S + s];
+      const int l = __ldcg(loc + k * S + s);
+      const bool kept = l < capacity;
+      const float g = kept ? gates[(int64_t)s * E + e] : 0.f;
+      weights[k * S + s] = g / denom;
+      ec_idx[k * S + s] = kept && g > 0.f ? e * capacity + l : (kept ? l : 0);
+    }
+  }
+  // Capacity slots no choice filled are given the lowest-numbered tokens that did not choose the expert
+  // within capacity; they carry no weight (the reference fills them with arbitrary zero-valued tokens).
+  // One warp per expert, 32 tokens at a time.
+  for (int e = sort.rank * SORT_WARPS + warp; e < E; e += sort.ctas * SORT_WARPS) {
+    int out = min(sort.count[e], capacity);
+    for (int t0 = 0; t0 < S && out < capacity; t0 += 32) {
+      const int t = t0 + lane;
+      bool open = t < S;
+      if (open) {
+#pragma unroll 4
+        for (int k = 0; k < K; ++k)
+          if (ids_km[k * S + t] == e && __ldcg(loc + k * S + t) < capacity) open = false;
+      }
+      const unsigned mask = __ballot_sync(0xffffffffu, open);
+      const int at = out + __popc(mask & ((1u << lane) - 1u));
+      if (open && at < capacity) select[(int64_t)e * capacity + at] = t;
+      out += __popc(mask);
+    }
+  }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.f;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
-    l_aux[0] = t / (float)E * (float)E * (float)E;
-  }
+  cl.sync();          // rank 0 has read the others' shared memory
 }
-// Queue position of every (choice, token) slot and the per-expert token lists.
-__global__ void __launch_bounds__(256) gshard_queue_kernel(const int32_t* __restrict__ sorted_slots,
-                                                           const int32_t* __restrict__ prefix,
-                                                           const int32_t* __restrict__ ids_km,
-                                                           int32_t* __restrict__ loc, int64_t* __restrict__ select,
-                                                           int64_t KS, int64_t S, int E, int capacity) {
-  for (int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; p < KS; p += (int64_t)gridDim.x * blockDim.x) {
-    const int slot = sorted_slots[p];
-    const int e = ids_km[slot];
-    const int l = (int)p - prefix[e];
-    loc[slot] = l;
-    if (l < capacity) select[(int64_t)e * capacity + l] = slot % S;   // token of the l-th kept choice
+static int launch_gshard_assign(const float* gates, const int32_t* ids_km, const float* part, int64_t rows,
+                                int32_t* loc, float* me, float* ce, float* l_aux, int32_t* ec_idx, float* weights,
+                                int64_t* select, int64_t tokens, int experts, int top_k, int64_t capacity,
+                                cudaStream_t stream) {
+  const size_t smem = sizeof(int32_t) * (sort_smem_ints(experts) + 2 * (size_t)experts);
+  const cudaError_t e = launch_one_cluster(gshard_assign_kernel, sort_cluster_size(tokens * top_k), smem, stream, gates,
+                                           ids_km, part, (int)rows, loc, me, ce, l_aux, ec_idx, weights, select,
+                                           (int)tokens, experts, top_k, (int)capacity, 1.1920928955078125e-07f);
+  if (e != cudaSuccess) {
+    set_last_error("gshard_assign: launch: %s", cudaGetErrorString(e));
+    return (int)e;
   }
-}
-// Capacity slots no choice filled are given the lowest-numbered tokens that did not choose the expert
-// within capacity; they carry no weight (the reference fills them with arbitrary zero-valued tokens).
-__global__ void __launch_bounds__(256) gshard_fill_kernel(const int32_t* __restrict__ prefix,
-                                                          int64_t* __restrict__ select, int E, int capacity,
-                                                          int64_t S) {
-  const int e = blockIdx.x;
-  const int kept = min(prefix[e + 1] - prefix[e], capacity);
-  // the kept tokens of this expert, as a bitmap in shared memory
-  extern __shared__ uint32_t bits[];
-  const int words = (int)((S + 31) / 32);
-  for (int w = threadIdx.x; w < words; w += blockDim.x) bits[w] = 0;
-  __syncthreads();
-  for (int i = threadIdx.x; i < kept; i += blockDim.x) {
-    const int64_t t = select[(int64_t)e * capacity + i];
-    atomicOr(&bits[t >> 5], 1u << (t & 31));
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int out = kept;
-    for (int64_t t = 0; t < S && out < capacity; ++t)
-      if (!((bits[t >> 5] >> (t & 31)) & 1u)) select[(int64_t)e * capacity + out++] = t;
-  }
-}
-// Per token: drop choices beyond capacity, normalise the kept gate values, emit e * capacity + position.
-__global__ void __launch_bounds__(256) gshard_assign_kernel(const float* __restrict__ gates,
-                                                            const int32_t* __restrict__ ids_km,
-                                                            const int32_t* __restrict__ loc,
-                                                            int32_t* __restrict__ ec_idx, float* __restrict__ weights,
-                                                            int64_t S, int E, int K, int capacity, float eps) {
-  const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= S) return;
-  float denom = 0.f;
-  for (int k = 0; k < K; ++k) {
-    const int e = ids_km[k * S + s];
-    if (loc[k * S + s] < capacity) denom += gates[s * E + e];
-  }
-  denom = fmaxf(denom, eps);
-  for (int k = 0; k < K; ++k) {
-    const int e = ids_km[k * S + s];
-    const int l = loc[k * S + s];
-    const bool kept = l < capacity;
-    const float g = kept ? gates[s * E + e] : 0.f;
-    weights[k * S + s] = g / denom;
-    ec_idx[k * S + s] = kept && g > 0.f ? e * capacity + l : (kept ? l : 0);
-  }
+  DLB_CUDA_LAUNCH_CHECK();
+  return DLB_OK;
 }
 // grad_logits[s, i] = g_i * (gg_i - sum_j g_j gg_j),  gg_e = grad_l_aux * ce[e] * E / S
 // (python/dlBLAS/dlblas/kernels/topk_gating_bwd.py:20-66)
@@ -761,41 +819,66 @@ extern "C" int dlb_gshard_assign(const float* gates, const int32_t* ids_choice_m
                                  int64_t* expert_select_token_idx, void* stream) {
   DLB_NVTX("dlb_gshard_assign");
   using namespace dlb;
+  (void)sorted_slots;       // the launch sorts the slots itself
+  (void)expert_prefix;
   DLB_CHECK_ARG(tokens >= 1 && experts >= 1 && experts <= 1024 && top_k >= 1 && capacity >= 1 && colsum_blocks >= 1,
                 DLB_ERR_BAD_ARG, "gshard_assign: bad sizes");
-  DLB_CHECK_ARG(tokens * top_k < (1LL << 31) && (int64_t)experts * capacity < (1LL << 31), DLB_ERR_TOO_LARGE,
+  DLB_CHECK_ARG(tokens * top_k < (1LL << 30) && (int64_t)experts * capacity < (1LL << 31), DLB_ERR_TOO_LARGE,
                 "gshard_assign: problem too large");
-  DLB_CHECK_ARG(gates && ids_choice_major && sorted_slots && expert_prefix && colsum_scratch && loc && me && ce &&
-                    l_aux && ec_idx && weights && expert_select_token_idx,
+  DLB_CHECK_ARG(gates && ids_choice_major && colsum_scratch && loc && me && ce && l_aux && ec_idx && weights &&
+                    expert_select_token_idx,
                 DLB_ERR_BAD_ARG, "gshard_assign: null pointer");
   cudaStream_t s = (cudaStream_t)stream;
   const int rows_per_block = (int)((tokens + colsum_blocks - 1) / colsum_blocks);
   gshard_colsum_stage1<<<(unsigned)colsum_blocks, 256, 0, s>>>(gates, colsum_scratch, tokens, experts, rows_per_block);
   DLB_CUDA_LAUNCH_CHECK();
-  gshard_aux_kernel<<<1, 256, experts * sizeof(float), s>>>(colsum_scratch, (int)colsum_blocks, ids_choice_major,
-                                                            tokens, experts, me, ce, l_aux);
-  DLB_CUDA_LAUNCH_CHECK();
-  const int64_t KS = tokens * top_k;
-  int64_t blocks = (KS + 255) / 256;
-  if (blocks > 4096) blocks = 4096;
-  gshard_queue_kernel<<<(unsigned)blocks, 256, 0, s>>>(sorted_slots, expert_prefix, ids_choice_major, loc,
-                                                       expert_select_token_idx, KS, tokens, experts, (int)capacity);
-  DLB_CUDA_LAUNCH_CHECK();
-  const size_t bitmap = (size_t)((tokens + 31) / 32) * 4;
-  DLB_CHECK_ARG(bitmap <= 200 * 1024, DLB_ERR_TOO_LARGE, "gshard_assign: more than 1.6M tokens");
-  cudaError_t e = cudaFuncSetAttribute(gshard_fill_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bitmap);
-  if (e != cudaSuccess) {
-    set_last_error("gshard_assign: smem attribute: %s", cudaGetErrorString(e));
-    return (int)e;
+  return launch_gshard_assign(gates, ids_choice_major, colsum_scratch, colsum_blocks, loc, me, ce, l_aux, ec_idx,
+                              weights, expert_select_token_idx, tokens, experts, top_k, capacity, s);
+}
+
+// Rows of column sums that dlb_gshard_forward writes: one per CTA of the gate kernel.
+static int64_t gshard_colsum_rows(int64_t tokens, int experts) {
+  const int warps = experts > 256 ? 4 : 8;      // GateShape<VPL>::WARPS
+  return (tokens + warps - 1) / warps;
+}
+
+extern "C" int dlb_gshard_forward(const float* logits, int64_t tokens, int experts, int top_k, int64_t capacity,
+                                  float* gates, int32_t* ids_choice_major, float* colsum_scratch,
+                                  int64_t colsum_floats, int32_t* loc, float* me, float* ce, float* l_aux,
+                                  int32_t* ec_idx, float* weights, int64_t* expert_select_token_idx, void* stream) {
+  DLB_NVTX("dlb_gshard_forward");
+  using namespace dlb;
+  DLB_CHECK_ARG(tokens >= 1 && experts >= 1 && experts <= 512 && top_k >= 1 && top_k <= 32 && top_k <= experts &&
+                    capacity >= 1,
+                DLB_ERR_BAD_ARG, "gshard_forward: bad sizes");
+  DLB_CHECK_ARG(tokens * top_k < (1LL << 30) && (int64_t)experts * capacity < (1LL << 31), DLB_ERR_TOO_LARGE,
+                "gshard_forward: problem too large");
+  DLB_CHECK_ARG(logits && gates && ids_choice_major && colsum_scratch && loc && me && ce && l_aux && ec_idx &&
+                    weights && expert_select_token_idx,
+                DLB_ERR_BAD_ARG, "gshard_forward: null pointer");
+  const int64_t rows = gshard_colsum_rows(tokens, experts);
+  DLB_CHECK_ARG(colsum_floats >= rows * experts, DLB_ERR_BAD_ARG, "gshard_forward: column-sum scratch holds %lld floats, needs %lld",
+                (long long)colsum_floats, (long long)(rows * experts));
+  int vpl = 1;
+  while (vpl * 32 < experts) vpl <<= 1;
+  if (vpl >= 4)
+    DLB_CHECK_ARG(((uintptr_t)logits & 15) == 0 && experts % 4 == 0, DLB_ERR_ALIGNMENT,
+                  "gshard_forward: logits rows must be 16-byte aligned");
+  GatingParams p{logits, nullptr, ids_choice_major, nullptr, gates, tokens, experts, experts, 1, 1, top_k,
+                 DLB_SCORE_SOFTMAX, 0, 1.0f};
+  p.colsum = colsum_scratch;
+  cudaStream_t s = (cudaStream_t)stream;
+  const unsigned g = (unsigned)rows, t = vpl >= 16 ? 128 : 256;
+  switch (vpl) {
+    case 1: grouped_topk_kernel<1, false, -1, 0, true><<<g, t, 0, s>>>(p); break;
+    case 2: grouped_topk_kernel<2, false, -1, 0, true><<<g, t, 0, s>>>(p); break;
+    case 4: grouped_topk_kernel<4, false, -1, 0, true><<<g, t, 0, s>>>(p); break;
+    case 8: grouped_topk_kernel<8, false, -1, 0, true><<<g, t, 0, s>>>(p); break;
+    default: grouped_topk_kernel<16, false, -1, 0, true><<<g, t, 0, s>>>(p); break;
   }
-  gshard_fill_kernel<<<(unsigned)experts, 256, bitmap, s>>>(expert_prefix, expert_select_token_idx, experts,
-                                                            (int)capacity, tokens);
   DLB_CUDA_LAUNCH_CHECK();
-  gshard_assign_kernel<<<(unsigned)((tokens + 255) / 256), 256, 0, s>>>(gates, ids_choice_major, loc, ec_idx, weights,
-                                                                        tokens, experts, top_k, (int)capacity,
-                                                                        1.1920928955078125e-07f);
-  DLB_CUDA_LAUNCH_CHECK();
-  return DLB_OK;
+  return launch_gshard_assign(gates, ids_choice_major, colsum_scratch, rows, loc, me, ce, l_aux, ec_idx, weights,
+                              expert_select_token_idx, tokens, experts, top_k, capacity, s);
 }
 
 extern "C" int dlb_gshard_gate_bwd(const float* gates, const float* ce, const float* grad_l_aux, float* grad_logits,

@@ -5,7 +5,6 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from .fused_moe import _moe_align
 
 
 def _capacity(num_tokens: int, num_experts: int, capacity_factor: float, min_capacity: int) -> int:
@@ -26,16 +25,10 @@ class TopKGatingFunc(torch.autograd.Function):
         x = logits.float().contiguous()
         lib = _lib.load()
         stream = _lib.stream_ptr(dev)
+        rows = (S + 3) // 4 if E > 256 else (S + 7) // 8              # column sums: one row per CTA of the gate kernel
         gates = torch.empty((S, E), dtype=torch.float32, device=dev)
-        ids = torch.empty((S, k), dtype=torch.int32, device=dev)
-        scratch_w = torch.empty((S, k), dtype=torch.float32, device=dev)
-        with torch.cuda.device(dev):
-            _lib.check(lib.dlb_gshard_gate(x.data_ptr(), S, E, k, gates.data_ptr(), ids.data_ptr(),
-                                           scratch_w.data_ptr(), stream), "topk_gating(gate)")
-        ids_km = ids.t().contiguous().view(-1)                        # choice-major: all first choices, then second, ...
-        sorted_ids, _, _, prefix = _moe_align(ids_km, 1, E)
-        nblk = max(1, min(256, S // 64))
-        colsum = torch.empty((nblk, E), dtype=torch.float32, device=dev)
+        colsum = torch.empty(rows * E, dtype=torch.float32, device=dev)
+        ids_km = torch.empty(k * S, dtype=torch.int32, device=dev)    # choice-major: all first choices, then second, ...
         loc = torch.empty(k * S, dtype=torch.int32, device=dev)
         me = torch.empty(E, dtype=torch.float32, device=dev)
         ce = torch.empty(E, dtype=torch.float32, device=dev)
@@ -44,11 +37,10 @@ class TopKGatingFunc(torch.autograd.Function):
         weights = torch.empty(k * S, dtype=torch.float32, device=dev)
         select = torch.empty(E * capacity, dtype=torch.int64, device=dev)
         with torch.cuda.device(dev):
-            _lib.check(lib.dlb_gshard_assign(gates.data_ptr(), ids_km.data_ptr(), sorted_ids.data_ptr(),
-                                             prefix.data_ptr(), S, E, k, capacity, colsum.data_ptr(), nblk,
-                                             loc.data_ptr(), me.data_ptr(), ce.data_ptr(), l_aux.data_ptr(),
-                                             ec_idx.data_ptr(), weights.data_ptr(), select.data_ptr(), stream),
-                       "topk_gating(assign)")
+            _lib.check(lib.dlb_gshard_forward(x.data_ptr(), S, E, k, capacity, gates.data_ptr(), ids_km.data_ptr(),
+                                              colsum.data_ptr(), colsum.numel(), loc.data_ptr(), me.data_ptr(),
+                                              ce.data_ptr(), l_aux.data_ptr(), ec_idx.data_ptr(), weights.data_ptr(),
+                                              select.data_ptr(), stream), "topk_gating")
         ctx.out_dtype = logits.dtype
         ctx.higher_precision = bool(higher_precision)
         ctx.mark_non_differentiable(ec_idx, select)

@@ -66,14 +66,16 @@ int dlb_grouped_topk_gating(const float* logits, const float* bias, int32_t* ids
  * topk_gating_bwd.py:20-85; torch statement python/dlBLAS/benchmarks/topk_gating.py:132-206.
  *   dlb_gshard_gate     gates = softmax(logits) [tokens, experts] fp32 and the k largest experts per token
  *                       (ids [tokens, top_k], descending, ties to the lower index).
- *   dlb_gshard_assign   from the choice-major id list [top_k * tokens] and its stable sort by expert
- *                       (dlb_moe_align_block_size with block 1): queue position of every choice (loc),
+ *   dlb_gshard_assign   from the choice-major id list [top_k * tokens]: queue position of every choice (loc),
  *                       me / ce / l_aux = mean(me * ce) * E^2, kept choices (position < capacity),
  *                       weights = kept gate / max(sum of the token's kept gates, fp32 eps),
  *                       ec_idx = expert * capacity + position (0 when dropped),
  *                       expert_select_token_idx [experts * capacity] int64 = tokens of each expert's queue
  *                       in arrival order, unfilled capacity padded with unrelated zero-weight tokens.
- *                       colsum_scratch: fp32 [colsum_blocks * experts].
+ *                       colsum_scratch: fp32 [colsum_blocks * experts].  sorted_slots and expert_prefix
+ *                       are not read any more (may be NULL): the launch sorts the slots itself.
+ *   dlb_gshard_forward  both in two launches, ids choice-major; colsum_scratch: fp32, at least
+ *                       ceil(tokens / 8) * experts of them (ceil(tokens / 4) above 256 experts).
  *   dlb_gshard_gate_bwd grad_logits = softmax backward of grad_l_aux * ce * E / tokens. */
 int dlb_gshard_gate(const float* logits, int64_t tokens, int experts, int top_k, float* gates, int32_t* ids,
                     float* scratch_weights, void* stream);
@@ -81,6 +83,10 @@ int dlb_gshard_assign(const float* gates, const int32_t* ids_choice_major, const
                       const int32_t* expert_prefix, int64_t tokens, int experts, int top_k, int64_t capacity,
                       float* colsum_scratch, int64_t colsum_blocks, int32_t* loc, float* me, float* ce, float* l_aux,
                       int32_t* ec_idx, float* weights, int64_t* expert_select_token_idx, void* stream);
+int dlb_gshard_forward(const float* logits, int64_t tokens, int experts, int top_k, int64_t capacity, float* gates,
+                       int32_t* ids_choice_major, float* colsum_scratch, int64_t colsum_floats, int32_t* loc,
+                       float* me, float* ce, float* l_aux, int32_t* ec_idx, float* weights,
+                       int64_t* expert_select_token_idx, void* stream);
 int dlb_gshard_gate_bwd(const float* gates, const float* ce, const float* grad_l_aux, float* grad_logits,
                         int64_t tokens, int experts, void* stream);
 /* Backward of topk_gating's `higher_precision` mode (python/dlBLAS/dlblas/kernels/topk_gating.py:145-256,
