@@ -53,6 +53,8 @@ constexpr int KV_BOX = BN * 128;  // one 64-wide column box of a K or V tile
 constexpr int KV_STAGES = 2;
 constexpr int TMEM_COLS = 256;    // S0 [0,64) S1 [64,128) O [128,128+D)
 constexpr float RESCALE_THRESHOLD = 8.0f;   // log2 units
+constexpr int64_t L2_BYTES = 126 << 20;
+enum { ORDER_GROUPS, ORDER_SORTED, ORDER_TILES, ORDER_RAGGED };
 // (Computing a share of the exponentials with a degree-3 polynomial on the FMA pipe instead of the SFU,
 // as large kernels of this kind do, was measured on B200 at 12.5 %, 25 % and 37.5 % of the scores and
 // was 2 %, 4 % and 10 % slower on the 4 x 8192 benchmark: the softmax warps are bound by issue slots
@@ -138,6 +140,7 @@ struct PrefillParams {
   int batch, hq, hkv, group;
   int max_tiles;
   int causal;
+  int order;                      // of the CTAs, see prefill_tile
   float scale_log2;               // sm_scale * log2(e)
   uint32_t idesc_qk, idesc_pv;
   uint32_t v_lbo, v_sbo;          // MN-major descriptor strides of the V tile
@@ -169,6 +172,69 @@ __device__ __forceinline__ int table_entry(const void* t, int64_t i, int is64) {
   return is64 ? (int)reinterpret_cast<const int64_t*>(t)[i] : reinterpret_cast<const int32_t*>(t)[i];
 }
 
+// CTA index -> (sequence, row tile, q head); false if the CTA has no work.  Every warp works it out by itself.
+//   ORDER_GROUPS      (sequence, kv head) groups one after the other, inside a group the heavy (late, causal) tiles
+//                     first, the q heads of the group adjacent.  The CTAs resident at any time then share the K/V of one
+//                     or two groups (4 MiB each at 8k tokens), which stay in L2 instead of being re-read from HBM.
+//   ORDER_SORTED      the same with the sequences by descending key count: a long history must not start last.
+//   ORDER_TILES       the row tile slowest, so that the heavy tiles of all groups come first and the launch ends on
+//                     light ones; for K/V that stay in L2 altogether.
+//   ORDER_RAGGED      ORDER_TILES over the tiles that exist, the CTAs without work last: on 13 prompts of 17 to 901
+//                     tokens half the CTAs of the full grid have none, and spread over it they cost 13 us of 95.
+// The sorted forms keep one sequence per lane (batch <= 32).  Measured on B200, 32 / 8 heads of 128, causal, together
+// with the early first loads and the staged epilogue, before -> after: 1 x 2048 tokens 58 -> 47 us, 1 x 8192 512 -> 470,
+// 8 x 2048 328 -> 303, 8 x 256 20.2 -> 18.6, the 13 prompts 95 -> 88; four chunks of 256-768 tokens over 1000-8000
+// cached ones 249 -> 235.  16 x 64 tokens, all in flight at once, 12.3 -> 12.9.
+__device__ __forceinline__ bool prefill_tile(const PrefillParams& p, int x, int& seq, int& tile, int& head) {
+  if (p.order == fp::ORDER_GROUPS) {
+    const int hig = x % p.group;
+    x /= p.group;
+    tile = p.max_tiles - 1 - x % p.max_tiles;
+    x /= p.max_tiles;
+    head = x % p.hkv * p.group + hig;
+    seq = x / p.hkv;
+    return true;
+  }
+  if (p.order == fp::ORDER_TILES) {
+    head = x % p.hq;
+    x /= p.hq;
+    seq = x % p.batch;
+    tile = p.max_tiles - 1 - x / p.batch;
+    return true;
+  }
+  const int lane = threadIdx.x & 31;
+  const int mine = lane < p.batch ? (p.paged ? p.kv_seq_len : p.b_seq_len)[lane] : -1;
+  int place = 0;                       // this lane's sequence among the lengths in descending order
+  for (int j = 0; j < p.batch; ++j) {
+    const int v = __shfl_sync(0xffffffffu, mine, j);
+    place += v > mine || (v == mine && j < lane) ? 1 : 0;
+  }
+  int turn;
+  if (p.order == fp::ORDER_SORTED) {
+    const int hig = x % p.group;
+    x /= p.group;
+    tile = p.max_tiles - 1 - x % p.max_tiles;
+    x /= p.max_tiles;
+    head = x % p.hkv * p.group + hig;
+    turn = x / p.hkv;
+  } else {
+    // at tile t the sequences with more than t tiles are the first ones of the sorted order
+    const int tiles = min(p.max_tiles, (mine + fp::BM - 1) / fp::BM);
+    int t = __reduce_max_sync(0xffffffffu, tiles) - 1;
+    for (; t >= 0; --t) {
+      const int n = __popc(__ballot_sync(0xffffffffu, tiles > t)) * p.hq;
+      if (x < n) break;
+      x -= n;
+    }
+    if (t < 0) return false;
+    tile = t;
+    turn = x / p.hq;
+    head = x - turn * p.hq;
+  }
+  seq = __ffs(__ballot_sync(0xffffffffu, lane < p.batch && place == turn)) - 1;
+  return true;
+}
+
 template <typename T, int D, bool EXTRAS>
 __global__ void __launch_bounds__(fp::THREADS, 2)
 flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
@@ -178,31 +244,24 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   constexpr int BOXES = L::BOXES;
   constexpr int Q_BYTES = L::Q_BYTES, KV_BYTES = L::KV_BYTES;
   constexpr int OFF_Q = L::OFF_Q, OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_CTRL = L::OFF_CTRL;
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
   // ---- which tile ----
-  // CTA order: (sequence, kv head) groups one after the other; inside a group the heavy (late, causal)
-  // tiles first, the q heads of the group adjacent.  The CTAs resident at any time then share the K/V
-  // of one or two groups (4 MiB each at 8k tokens), which stay in L2 instead of being re-read from HBM.
-  int x = blockIdx.x;
-  const int hig = x % p.group;
-  x /= p.group;
-  const int tile = p.max_tiles - 1 - x % p.max_tiles;
-  x /= p.max_tiles;
-  const int kvh_ = x % p.hkv;
-  const int seq = x / p.hkv;
-  const int head = kvh_ * p.group + hig;
+  int seq, tile, head;
+  if (!prefill_tile(p, (int)blockIdx.x, seq, tile, head)) return;
+  const int kvh = head / p.group;
   const int seq_len = p.b_seq_len[seq];
+  const int start = p.b_start_loc[seq];
+  const int kv_len = p.paged ? p.kv_seq_len[seq] : seq_len;
   const int q0 = tile * BM;
   if (q0 >= seq_len) return;
-  const int start = p.b_start_loc[seq];
   // query row r of the tile sits at position hist + q0 + r of its sequence (hist = tokens already cached)
-  const int kv_len = p.paged ? p.kv_seq_len[seq] : seq_len;
   const int hist = kv_len - seq_len;
   const int kv_end = p.causal ? min(kv_len, q0 + BM + hist) : kv_len;
   // with a sliding window the tile starts at the block that holds the first key its first row may see;
   // `j` below counts blocks from there, jb0 + j is the block's index in the sequence
   const int jb0 = (EXTRAS && p.window > 0) ? max(0, q0 + hist - p.window) / BN : 0;
   const int nb = (kv_end + BN - 1) / BN - jb0;
-  const int kvh = head / p.group;
 
   extern __shared__ __align__(1024) uint8_t smem[];
   if ((smem_u32(smem) & 1023u) != 0) {
@@ -223,10 +282,45 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-
-  if (threadIdx.x == 0) {
+  // ------------------------------ TMA producer (one lane) ------------------------------
+  // paged: the 64 keys of block j come from 64 / min(page, 64) pages of this sequence's table.  The table entries
+  // of block j + 1 are fetched right after block j's K loads are issued, so that the look-up's latency never sits
+  // between a freed stage and its next load.
+  const int box_slots = min(p.page_size, BN);
+  const int n_sub = p.paged ? BN / box_slots : 0;
+  int pg[4] = {0, 0, 0, 0}, sl[4] = {0, 0, 0, 0};
+  auto look_up = [&](int j) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (u >= n_sub) break;
+      const int tok = (jb0 + j) * BN + u * box_slots;
+      int page_slot = tok / p.page_size;
+      if (page_slot >= p.max_pages) page_slot = p.max_pages - 1;   // past the table: any valid page, masked later
+      int page = table_entry(p.block_table, (int64_t)seq * p.bt_stride + page_slot, p.table_is_int64);
+      if (tok >= kv_len || page < 0 || page >= p.num_pages) page = 0;
+      pg[u] = page;
+      sl[u] = tok % p.page_size;
+    }
+  };
+  auto load_block = [&](int j, int off, const CUtensorMap* tmap, uint64_t* full, const int (&page)[4],
+                        const int (&slot)[4]) {
+    uint8_t* dst = smem + off + (j & 1) * KV_BYTES;
+    mbar_arrive_expect_tx(&full[j & 1], KV_BYTES);
+    if (p.paged) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (u >= n_sub) break;
+#pragma unroll
+        for (int bx = 0; bx < BOXES; ++bx)
+          tma_load_4d(dst + bx * KV_BOX + u * box_slots * 128, tmap, &full[j & 1], bx * 64, kvh, slot[u], page[u]);
+      }
+    } else {
+#pragma unroll
+      for (int bx = 0; bx < BOXES; ++bx)
+        tma_load_3d(dst + bx * KV_BOX, tmap, &full[j & 1], bx * 64, kvh, start + (jb0 + j) * BN);
+    }
+  };
+  if (warp == WARP_TMA && lane == 0) {
     mbar_init(q_full, 1);
     mbar_init(q_ready, 128);
     for (int i = 0; i < 2; ++i) {
@@ -238,6 +332,16 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
     *abort_flag = 0;
     fence_mbar_init();
+    // Q and the first K and V block are on their way while the rest of the CTA sets up
+    mbar_arrive_expect_tx(q_full, Q_BYTES);
+#pragma unroll
+    for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(smem + OFF_Q + bx * Q_BOX, &tmap_q, q_full, bx * 64, head, start + q0);
+    if (nb > 0) {
+      look_up(0);
+      load_block(0, OFF_K, &tmap_k, k_full, pg, sl);
+      load_block(0, OFF_V, &tmap_v, v_full, pg, sl);
+      if (nb > 1) look_up(1);
+    }
   }
   if (warp == WARP_MMA) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -250,38 +354,10 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   const uint32_t tmem_o = tmem_base + 128;
 
   if (warp == WARP_TMA) {
-    // ------------------------------ TMA producer ------------------------------
     if (lane == 0) {
-      tma_prefetch_desc(&tmap_q);
-      tma_prefetch_desc(&tmap_k);
-      tma_prefetch_desc(&tmap_v);
-      mbar_arrive_expect_tx(q_full, Q_BYTES);
-#pragma unroll
-      for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(smem + OFF_Q + bx * Q_BOX, &tmap_q, q_full, bx * 64, head, start + q0);
-      // paged: the 64 keys of block j come from 64 / min(page, 64) pages of this sequence's table.  The
-      // table entries of block j + 1 are fetched right after block j's K loads are issued, so that the
-      // look-up's latency never sits between a freed stage and its next load.
-      const int box_slots = min(p.page_size, BN);
-      const int n_sub = p.paged ? BN / box_slots : 0;
-      int pg[4] = {0, 0, 0, 0}, sl[4] = {0, 0, 0, 0};
-      auto look_up = [&](int j) {
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          if (u >= n_sub) break;
-          const int tok = (jb0 + j) * BN + u * box_slots;
-          int page_slot = tok / p.page_size;
-          if (page_slot >= p.max_pages) page_slot = p.max_pages - 1;   // past the table: any valid page, masked later
-          int page = table_entry(p.block_table, (int64_t)seq * p.bt_stride + page_slot, p.table_is_int64);
-          if (tok >= kv_len || page < 0 || page >= p.num_pages) page = 0;
-          pg[u] = page;
-          sl[u] = tok % p.page_size;
-        }
-      };
-      if (nb > 0) look_up(0);
-      for (int j = 0; j < nb; ++j) {
+      for (int j = 1; j < nb; ++j) {
         const int s = j & 1;
         const uint32_t ph = (j >> 1) & 1;
-        const int row = start + (jb0 + j) * BN;
         int pv[4], sv[4];   // block j's pages for the V loads below
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
@@ -291,36 +367,10 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // K stage s is free once the Q K^T of block j - 2 has retired (s_full), V stage s once its P V has
         // (pv_done): no separate "empty" commits, every commit costs the single issuing thread ~100 clocks
         if (!mbar_wait(&s_full[s], ph ^ 1, abort_flag, p.status, 21, j)) break;
-        uint8_t* kd = smem + OFF_K + s * KV_BYTES;
-        mbar_arrive_expect_tx(&k_full[s], KV_BYTES);
-        if (p.paged) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (u >= n_sub) break;
-#pragma unroll
-            for (int bx = 0; bx < BOXES; ++bx)
-              tma_load_4d(kd + bx * KV_BOX + u * box_slots * 128, &tmap_k, &k_full[s], bx * 64, kvh, sl[u], pg[u]);
-          }
-        } else {
-#pragma unroll
-          for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(kd + bx * KV_BOX, &tmap_k, &k_full[s], bx * 64, kvh, row);
-        }
+        load_block(j, OFF_K, &tmap_k, k_full, pg, sl);
         if (j + 1 < nb) look_up(j + 1);
         if (!mbar_wait(&pv_done[s], ph ^ 1, abort_flag, p.status, 22, j)) break;
-        uint8_t* vd = smem + OFF_V + s * KV_BYTES;
-        mbar_arrive_expect_tx(&v_full[s], KV_BYTES);
-        if (p.paged) {
-#pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            if (u >= n_sub) break;
-#pragma unroll
-            for (int bx = 0; bx < BOXES; ++bx)
-              tma_load_4d(vd + bx * KV_BOX + u * box_slots * 128, &tmap_v, &v_full[s], bx * 64, kvh, sv[u], pv[u]);
-          }
-        } else {
-#pragma unroll
-          for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(vd + bx * KV_BOX, &tmap_v, &v_full[s], bx * 64, kvh, row);
-        }
+        load_block(j, OFF_V, &tmap_v, v_full, pv, sv);
       }
     }
   } else if (warp == WARP_MMA) {
@@ -573,26 +623,38 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       tc_fence_after_sync();
       const float inv_l = 1.f / l_sum;
       const bool row_ok = q_pos < seq_len;
-      T* orow = reinterpret_cast<T*>(p.out) + (int64_t)(start + q_pos) * p.o_stride_t + (int64_t)head * p.o_stride_h;
+      // Through the Q tile's shared memory (every Q K^T has retired; row r of O over row r of Q, same swizzle), so that
+      // the lanes of a store cover whole rows instead of 16 bytes of 32 rows each.
+      uint8_t* stage = smem + OFF_Q;
+      const int rows = min(32, seq_len - q0 - quad * 32);   // the warp's rows inside the sequence
 #pragma unroll 1
-      for (int c = 0; c < D / 32; ++c) {
-        uint32_t o[32];
-        tmem_ld_32x32b_x32(tmem_o + lane_field + c * 32, o);
+      for (int c = 0; rows > 0 && c < D / 64; ++c) {
+        uint32_t o[2][32];
+        tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64, o[0]);
+        tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64 + 32, o[1]);
         tmem_wait_ld();
-        if (row_ok) {
 #pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            uint32_t w[4];
+        for (int v = 0; v < 8; ++v) {
+          uint32_t w[4];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              typename Elem<T>::T2 v2 = Elem<T>::from_f2(__uint_as_float(o[v * 8 + 2 * i]) * inv_l,
-                                                         __uint_as_float(o[v * 8 + 2 * i + 1]) * inv_l);
-              w[i] = *reinterpret_cast<uint32_t*>(&v2);
-            }
-            if (c * 32 + v * 8 < p.dv)
-              *reinterpret_cast<uint4*>(orow + c * 32 + v * 8) = make_uint4(w[0], w[1], w[2], w[3]);
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t* pair = &o[v >> 2][(v & 3) * 8 + 2 * i];
+            typename Elem<T>::T2 v2 = Elem<T>::from_f2(__uint_as_float(pair[0]) * inv_l, __uint_as_float(pair[1]) * inv_l);
+            w[i] = *reinterpret_cast<uint32_t*>(&v2);
           }
+          *reinterpret_cast<uint4*>(stage + c * Q_BOX + row * 128 + ((v ^ (row & 7)) << 4)) =
+              make_uint4(w[0], w[1], w[2], w[3]);
         }
+      }
+      __syncwarp();
+      constexpr int LANES = D / 8;       // lanes per row
+      const int cc = lane % LANES;       // 16-byte chunk of the row
+      T* obase = reinterpret_cast<T*>(p.out) + (int64_t)head * p.o_stride_h + cc * 8;
+#pragma unroll 4
+      for (int i = lane / LANES; i < rows; i += 32 / LANES) {
+        const int r = quad * 32 + i;
+        const uint4 val = *reinterpret_cast<const uint4*>(stage + (cc >> 3) * Q_BOX + r * 128 + (((cc & 7) ^ (r & 7)) << 4));
+        if (cc * 8 < p.dv) *reinterpret_cast<uint4*>(obase + (int64_t)(start + q0 + r) * p.o_stride_t) = val;
       }
       if (row_ok && p.lse != nullptr) {
         p.lse[(int64_t)head * p.total_tokens + start + q_pos] = m_ref * 0.6931471805599453f + __logf(l_sum);
@@ -691,6 +753,13 @@ extern "C" int dlb_flash_prefill_varlen(const void* q, const void* k, const void
   p.v_lbo = KV_BOX;
   p.v_sbo = 1024;
   p.status = status;
+  // K/V of the launch stay in L2 (126 MB) when they take at most three quarters of it; sequences count as ragged when the full
+  // grid has a quarter more row tiles than the tokens can fill
+  p.order = ORDER_GROUPS;
+  if (total_tokens * hkv * (head_dim + head_dim_v) * 2 <= L2_BYTES / 4 * 3) {
+    const bool ragged = max_tiles * batch * 4 > (total_tokens / BM + batch) * 5;
+    p.order = !ragged ? ORDER_TILES : batch <= 32 ? ORDER_RAGGED : ORDER_GROUPS;
+  }
   p.paged = 0;
   p.page_size = BN;
   p.num_pages = p.max_pages = 0;
@@ -794,6 +863,8 @@ extern "C" int dlb_flash_prefill_paged(const void* q, const void* k_cache, const
   p.v_lbo = KV_BOX;
   p.v_sbo = 1024;
   p.status = status;
+  // a launch that starts all its CTAs at once gains nothing from their order
+  p.order = batch > 1 && batch <= 32 && grid > 2 * sm_count(current_device()) ? ORDER_SORTED : ORDER_GROUPS;
   p.paged = 1;
   p.page_size = (int)page_size;
   p.num_pages = (int)num_pages;
