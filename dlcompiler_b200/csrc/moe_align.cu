@@ -67,14 +67,16 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_align_kernel(
   sort.finish();
 }
 
-// dst[p, :] = src[sorted_token_ids[p] / top_k, :]  (zeros for sentinel rows).
+// dst[p, :] = src[sorted_token_ids[p] / top_k, :].  Sentinel rows become zeros, or are left alone when they are a large
+// share of the list (`zero_padding`; no GEMM stores what comes of them): with 256 experts of 62 rows in blocks of 128 they
+// were half the bytes written.
 // 16-byte vectors; one warp per row chunk keeps the accesses coalesced.
 __global__ void __launch_bounds__(256) moe_permute_rows_kernel(const uint4* __restrict__ src,
                                                                uint4* __restrict__ dst,
                                                                const int32_t* __restrict__ sorted_token_ids,
                                                                const int32_t* __restrict__ num_post_padded,
                                                                int numel, int top_k, int row_vecs,
-                                                               int64_t src_row_vecs, int sorted_capacity) {
+                                                               int64_t src_row_vecs, int sorted_capacity, int zero_padding) {
   const int rows = min(num_post_padded[0], sorted_capacity);
   for (int p = blockIdx.x; p < rows; p += gridDim.x) {
     const int sid = sorted_token_ids[p];
@@ -82,7 +84,7 @@ __global__ void __launch_bounds__(256) moe_permute_rows_kernel(const uint4* __re
     if (sid < numel) {
       const uint4* s = src + (int64_t)(sid / top_k) * src_row_vecs;
       for (int v = threadIdx.x; v < row_vecs; v += blockDim.x) d[v] = __ldg(s + v);
-    } else {
+    } else if (zero_padding) {
       for (int v = threadIdx.x; v < row_vecs; v += blockDim.x) d[v] = make_uint4(0, 0, 0, 0);
     }
   }
@@ -253,7 +255,8 @@ extern "C" int dlb_moe_permute_rows(const void* src, void* dst, const int32_t* s
   if (blocks > cap) blocks = cap;
   moe_permute_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
       (const uint4*)src, (uint4*)dst, sorted_token_ids, num_tokens_post_padded, (int)numel, top_k,
-      (int)(row_bytes / 16), src_row_stride * elem_size / 16, (int)sorted_capacity);
+      (int)(row_bytes / 16), src_row_stride * elem_size / 16, (int)sorted_capacity,
+      (sorted_capacity - numel) * 2 < numel ? 1 : 0);      // the grouped GEMM's rule for whole boxes of A
   DLB_CUDA_LAUNCH_CHECK();
   return DLB_OK;
 }
