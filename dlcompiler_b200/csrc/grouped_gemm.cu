@@ -100,11 +100,27 @@ template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) 
 }
 template <typename T> __device__ __forceinline__ float round_to(float a) { return Elem<T>::to_f(Elem<T>::from_f(a)); }
 
+// x / (1 + e^-x), the quotient from an approximate reciprocal and one residual correction (Newton-Raphson on the
+// quotient, as in Markstein's division), without a branch.  An IEEE division per element, with its branch for the ends
+// of the range, kept the 32 elements of a step from overlapping: the epilogue of a tile took about 55 000 clocks, and
+// every gate/up launch with a shorter main loop waited for it (32 experts, K = 1024: 235 us for 369 MB of weights).
+// Whole fused_moe, before -> after: 2000 tokens over 256 experts (2048 x 1024) 676 -> 600 us, 128 over 64 (2048 x 1408)
+// 246 -> 203, 32 over 32 (1024 x 2816) 195 -> 113, 4096 over 8 (4096 x 14336) 2394 -> 2298; same outputs bit for bit.
+// Both sides are scaled by 1/4 so that the reciprocal of the largest 1 + e^-x is not subnormal.
+__device__ __forceinline__ float silu_branchless(float x) {
+  const float d = fmaf(fminf(__expf(-x), 3.402823466e38f), 0.25f, 0.25f), a = x * 0.25f;
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+  const float q = a * r;
+  const float s = fmaf(fmaf(-q, d, a), r, q);
+  return x > 3.402823466e38f ? x : s;      // +inf; the correction would make it NaN (as the division does for -inf)
+}
+
 // silu(gate) * up with the reference's rounding points.
 template <typename T> __device__ __forceinline__ float silu_mul_rounded(float gate_acc, float up_acc) {
   const float g = round_to<T>(gate_acc);
   const float u = round_to<T>(up_acc);
-  const float s = round_to<T>(g / (1.0f + __expf(-g)));
+  const float s = round_to<T>(silu_branchless(g));
   return s * u;  // rounded by the caller's pack
 }
 

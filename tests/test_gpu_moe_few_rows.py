@@ -29,3 +29,21 @@ def test_rows_and_widths(cuda_device, rows, hidden, inter, dtype):
     ref = oracle.fused_moe_rounding_faithful(x, w1, w2, weights, ids)
     # stated bound of the block in 16 bits: 4 ulp of bf16 against the rounding-faithful oracle
     torch.testing.assert_close(out.cpu().float(), ref.float(), rtol=2e-2, atol=2e-2 * float(ref.float().std()))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_silu_over_its_range(cuda_device, dtype):
+    """The activation from one end of its range to the other: hidden state 1, gate weights the values, up weights 1 and
+    an identity behind it give silu(value).  Two roundings to the type; below 2^-24 only the size is left to compare."""
+    values = torch.cat([torch.linspace(-104, 104, 833), torch.tensor([-6e4, -500., -88.8, -87.4, 0., 1e-4, 500., 6e4])])
+    n = values.numel() // 8 * 8
+    values = values[-n:].to(dtype)
+    w1 = torch.zeros(1, 2 * n, 8)
+    w1[0, :n, 0], w1[0, n:, 0] = values.float(), 1.0
+    x = torch.zeros(1, 8)
+    x[0, 0] = 1.0
+    one = torch.ones(1, 1, device=cuda_device)
+    out = fused_moe(x.to(dtype).to(cuda_device), w1.to(dtype).to(cuda_device),
+                    torch.eye(n).unsqueeze(0).to(dtype).to(cuda_device), one, one.long() * 0, 1)
+    ref = torch.nn.functional.silu(values.double())
+    torch.testing.assert_close(out[0].cpu().double(), ref, rtol=2 * torch.finfo(dtype).eps, atol=2.0 ** -24)
