@@ -78,7 +78,7 @@ class CudaOps:
             ids = ids.to(torch.int64)
         ids = ids.contiguous()
         lib = _lib.load()
-        with torch.cuda.device(partial.device):
+        with _lib.on_device(partial.device):
             rc = lib.dlb_moe_combine(partial.data_ptr(), out.data_ptr(), tokens, top_k, partial.size(1),
                                      out.stride(0), _lib.dtype_code(out), ids.data_ptr(),
                                      int(ids.dtype == torch.int64), 0, num_experts,
@@ -313,7 +313,7 @@ def ep_fused_moe_peer(ctx: EpPeerContext, hidden_states, w1_local, w2_local, top
     _, H_out, inter = w2_local.shape
     out = torch.empty((T, H_out), dtype=ctx.dtype, device=dev)
     flags_local = ctx.flags.data_ptr()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_ep_route(ids.data_ptr(), is64, numel, ctx.counts_tbl, ctx.flags_tbl, ctx.dest_pos.data_ptr(),
                               ctx.block_start.data_ptr(), ctx.num_post.data_ptr(), ctx.row_map.data_ptr(), rank, world,
                               ctx.num_experts, ctx.cap, epoch, ctx.status.data_ptr(), stream)

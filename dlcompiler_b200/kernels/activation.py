@@ -24,7 +24,7 @@ def silu_and_mul(gate_up: torch.Tensor, out: torch.Tensor = None):
         gate_up = gate_up.contiguous()
     assert out.stride(1) == 1 or N <= 1, "out must be contiguous along its last dimension"
     lib = _lib.load()
-    with torch.cuda.device(gate_up.device):
+    with _lib.on_device(gate_up.device):
         rc = lib.dlb_silu_and_mul(gate_up.data_ptr(), out.data_ptr(), M, N, gate_up.stride(0) if M > 1 else 2 * N,
                                   out.stride(0) if M > 1 else N, _lib.dtype_code(gate_up),
                                   _lib.stream_ptr(gate_up.device))

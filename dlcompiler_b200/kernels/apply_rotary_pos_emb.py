@@ -35,10 +35,10 @@ def apply_rotary_pos_emb(
     cos = cos.to(q.dtype).contiguous()
     sin = sin.to(q.dtype).contiguous()
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    qs, ks, qes, kes = q.stride(), k.stride(), q_embed.stride(), k_embed.stride()
+    with _lib.on_device(dev):
         rc = lib.dlb_apply_rotary(q.data_ptr(), k.data_ptr(), cos.data_ptr(), sin.data_ptr(), q_embed.data_ptr(),
-                                  k_embed.data_ptr(), tokens, q.size(-2), k.size(-2), dim, q.stride(0), q.stride(1),
-                                  k.stride(0), k.stride(1), q_embed.stride(0), q_embed.stride(1), k_embed.stride(0),
-                                  k_embed.stride(1), _lib.dtype_code(q), _lib.stream_ptr(dev))
+                                  k_embed.data_ptr(), tokens, q.size(-2), k.size(-2), dim, qs[0], qs[1], ks[0], ks[1],
+                                  qes[0], qes[1], kes[0], kes[1], _lib.dtype_code(q), _lib.stream_ptr(dev))
     _lib.check(rc, "apply_rotary_pos_emb")
     return q_embed, k_embed

@@ -50,7 +50,7 @@ def decode_attention_fwd(
     nfloats = lib.dlb_paged_decode_workspace_floats(batch, head, max(D, Dv), max_splits)
     partial = torch.empty(max(nfloats, 1), dtype=torch.float32, device=dev)
     status = _lib.status_word(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_paged_decode(
             q.data_ptr(), k_buffer.data_ptr(), v_buffer.data_ptr(), o.data_ptr(), table.data_ptr(), lens.data_ptr(),
             partial.data_ptr(), batch, head, hkv, D, Dv, 1, k_buffer.size(0), table.size(1),

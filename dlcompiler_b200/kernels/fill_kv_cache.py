@@ -52,14 +52,13 @@ def fill_kv_cache(
         assert kc.shape[0] == k_states.shape[0] and ks.shape == kc.shape, "cos / sin need one row per new token"
         dt = _lib.dtype_code(k_states)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    kst, vst, kct, vct = k_states.stride(), v_states.stride(), k_caches.stride(), v_caches.stride()
+    with _lib.on_device(dev):
         rc = lib.dlb_fill_kv_cache(
             k_states.data_ptr(), v_states.data_ptr(), k_caches.data_ptr(), v_caches.data_ptr(), q_start_loc.data_ptr(),
             q_seq_length.data_ptr(), kv_seq_length.data_ptr(), block_offsets.data_ptr(), batch_size,
             int(max_q_seq_length), block_size, num_heads, head_dim, head_dim_v, k_caches.size(0), block_offsets.size(1),
-            k_states.stride(-3), k_states.stride(-2), v_states.stride(-3), v_states.stride(-2),
-            k_caches.stride(0), k_caches.stride(1), k_caches.stride(2), v_caches.stride(0), v_caches.stride(1),
-            v_caches.stride(2), block_offsets.stride(0), _is64(q_start_loc), _is64(q_seq_length),
+            kst[-3], kst[-2], vst[-3], vst[-2], kct[0], kct[1], kct[2], vct[0], vct[1], vct[2], block_offsets.stride(0), _is64(q_start_loc), _is64(q_seq_length),
             _is64(kv_seq_length), _is64(block_offsets), k_states.element_size(), _lib.ptr(kc), _lib.ptr(ks), dt,
             _lib.stream_ptr(dev))
     _lib.check(rc, "fill_kv_cache")

@@ -33,7 +33,7 @@ def _moe_align(topk_ids: torch.Tensor, block: int, num_experts: int):
     num_post = meta[:1]
     block_start = meta[1:]
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_moe_align_block_size(ids.data_ptr(), int(ids.dtype == torch.int64), numel, num_experts, block,
                                           sorted_ids.data_ptr(), cap, expert_ids.data_ptr(), expert_ids.numel(),
                                           num_post.data_ptr(), block_start.data_ptr(), _lib.stream_ptr(dev))
@@ -59,7 +59,7 @@ def _permute_rows(src, row_map, num_post, numel, div, cap):
     hidden = src.size(-1)
     dst = torch.empty((cap, hidden), dtype=src.dtype, device=src.device)
     lib = _lib.load()
-    with torch.cuda.device(src.device):
+    with _lib.on_device(src.device):
         rc = lib.dlb_moe_permute_rows(src.data_ptr(), dst.data_ptr(), row_map.data_ptr(), num_post.data_ptr(), numel,
                                       div, hidden, src.stride(0), cap, src.element_size(),
                                       _lib.stream_ptr(src.device))
@@ -73,7 +73,7 @@ def _grouped_gemm(a, b, out, n_out, row_map, block_start, weights, numel, flags)
     assert a.stride(1) == 1 and out.stride(-1) == 1
     lib = _lib.load()
     status = _lib.status_word(a.device)
-    with torch.cuda.device(a.device):
+    with _lib.on_device(a.device):
         rc = lib.dlb_moe_grouped_gemm(a.data_ptr(), a.size(0), a.stride(0), b.data_ptr(), E, rows_per_expert, K,
                                       b.stride(1), out.data_ptr(), out.stride(0), n_out, row_map.data_ptr(),
                                       block_start.data_ptr(), _lib.ptr(weights), numel, flags,
@@ -141,7 +141,7 @@ def fused_moe(hidden_states: torch.Tensor,
     ids = topk_ids if topk_ids.dtype in (torch.int32, torch.int64) else topk_ids.to(torch.int64)
     ids = ids.contiguous()
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_moe_combine(partial.data_ptr(), out.data_ptr(), M, topk, H_out, out.stride(0),
                                  _lib.dtype_code(out), ids.data_ptr(), int(ids.dtype == torch.int64),
                                  expert_offset, expert_offset + E, _lib.stream_ptr(dev))
@@ -165,7 +165,7 @@ def get_start_end(topk_idx: torch.Tensor, sorted_idx: torch.Tensor, num_experts:
     out_dtype = torch.int64 if sorted_idx.dtype == torch.int64 else torch.int32
     start_end = torch.empty((2, num_experts), dtype=out_dtype, device=flat.device)
     lib = _lib.load()
-    with torch.cuda.device(flat.device):
+    with _lib.on_device(flat.device):
         rc = lib.dlb_moe_start_end(flat.data_ptr(), int(flat.dtype == torch.int64), flat.numel(), num_experts,
                                    start_end[0].data_ptr(), start_end[1].data_ptr(), int(out_dtype == torch.int64),
                                    _lib.stream_ptr(flat.device))

@@ -33,7 +33,7 @@ def fused_rotary_and_fa(q, k, v, cos, sin, causal=False, softmax_scale=None):
     sin2 = sin.to(q.dtype).reshape(tokens, d).contiguous()
     k_rot = torch.empty_like(k3)
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         # keys only: no query heads in this launch
         rc = lib.dlb_apply_rotary(None, k3.data_ptr(), cos2.data_ptr(), sin2.data_ptr(), None, k_rot.data_ptr(),
                                   tokens, 0, nheads, d, 0, 0, k3.stride(0), k3.stride(1), 0, 0, k_rot.stride(0),

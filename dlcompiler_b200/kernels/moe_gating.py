@@ -39,7 +39,7 @@ def grouped_topk_gating(logits: torch.Tensor, bias: torch.Tensor | None, top_k: 
     weights = torch.empty((T, top_k), dtype=torch.float32, device=logits.device)
     scoring = {"sigmoid": _lib.SCORE_SIGMOID, "softmax": _lib.SCORE_SOFTMAX}[scoring_func]
     lib = _lib.load()
-    with torch.cuda.device(logits.device):
+    with _lib.on_device(logits.device):
         rc = lib.dlb_grouped_topk_gating(logits.data_ptr(), _lib.ptr(bias), ids.data_ptr(), weights.data_ptr(), T, E,
                                          logits.stride(0) if T > 1 else E, n_group, topk_group, top_k, scoring,
                                          int(renormalize), float(routed_scaling_factor),

@@ -100,12 +100,12 @@ def paged_attention_fwd(
     nfloats = lib.dlb_paged_decode_workspace_floats(batch, head, max(Lq, Lv), max_splits)
     partial = torch.empty(max(nfloats, 1), dtype=torch.float32, device=dev)
     status = _lib.status_word(dev)
-    with torch.cuda.device(dev):
+    ks, vs, qs, os_ = k.stride(), v.stride(), q.stride(), o.stride()
+    with _lib.on_device(dev):
         rc = lib.dlb_paged_decode(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), block_offsets.data_ptr(), kv_seqlens.data_ptr(),
             partial.data_ptr(), batch, head, hkv, Lq, Lv, BLOCK, k.size(0), max_pages,
-            q.stride(-3), q.stride(-2), o.stride(-3), o.stride(-2),
-            k.stride(0), k.stride(1), k.stride(2), v.stride(0), v.stride(1), v.stride(2),
+            qs[-3], qs[-2], os_[-3], os_[-2], ks[0], ks[1], ks[2], vs[0], vs[1], vs[2],
             block_offsets.stride(0), int(block_offsets.dtype == torch.int64), int(kv_seqlens.dtype == torch.int64),
             chunk, max_splits, window_size, float(sm_scale), float(logit_softcapping), _lib.dtype_code(q),
             status.data_ptr(), _lib.stream_ptr(dev))
@@ -130,7 +130,7 @@ def _paged_prefill(q, k, v, o, block_offsets, q_start_loc, q_seqlens, kv_seqlens
     cos, sin = _rotary_tables(q, q_cos, q_sin)
     lib = _lib.load()
     status = _lib.status_word(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_flash_prefill_paged(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), None, block_offsets.data_ptr(),
             q_start.data_ptr(), q_len.data_ptr(), kv_len.data_ptr(), batch, q.shape[0], int(max_seqlen),

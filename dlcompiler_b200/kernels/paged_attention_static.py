@@ -44,7 +44,7 @@ def paged_decode_no_alloc(q: Tensor, k: Tensor, v: Tensor, o: Tensor, block_offs
     lib = _lib.load()
     # the status word is a torch tensor: use it only if an earlier call already made it (NULL is allowed)
     status = _lib.existing_status_word(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_paged_decode_static(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), block_offsets.data_ptr(), kv_seqlens.data_ptr(),
             batch, head, hkv, D, page, k.size(0), max_pages, q.stride(0), q.stride(1), o.stride(0), o.stride(1),

@@ -72,7 +72,7 @@ def context_attention_fwd(q, k, v, o, b_start_loc, b_seq_len, max_input_len, lse
     cos, sin = _rotary_tables(q, q_cos, q_sin)
     lib = _lib.load()
     status = _lib.status_word(dev)
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_flash_prefill_varlen(
             q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), _lib.ptr(lse), b_start_loc.data_ptr(),
             b_seq_len.data_ptr(), batch, q.shape[0], int(max_input_len), head, k.shape[1], Lq, Lv,

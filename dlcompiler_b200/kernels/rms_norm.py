@@ -19,7 +19,7 @@ def _launch(x, weight, residual, out, out_residual, eps, weight_after_cast):
     if r2 is not None and or2 is not None:
         assert r2.stride(0) == or2.stride(0), "residual and out_residual must share their row stride"
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with _lib.on_device(dev):
         rc = lib.dlb_rms_norm(x2.data_ptr(), weight.data_ptr(), _lib.ptr(r2), o2.data_ptr(), _lib.ptr(or2), rows, n,
                               x2.stride(0) if rows > 1 else n, (r2.stride(0) if rows > 1 else n) if r2 is not None else n,
                               o2.stride(0) if rows > 1 else n, float(eps), int(weight_after_cast), _lib.dtype_code(x),

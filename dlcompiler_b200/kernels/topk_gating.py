@@ -2,15 +2,22 @@
 (python/dlBLAS/dlblas/__init__.py:13-23, python/dlBLAS/dlblas/kernels/topk_gating.py:259-294)."""
 from __future__ import annotations
 
+import ctypes
+import math
+
 import torch
 
 from .. import _lib
 
 
+def _f32(x: float) -> float:
+    return ctypes.c_float(x).value
+
+
 def _capacity(num_tokens: int, num_experts: int, capacity_factor: float, min_capacity: int) -> int:
     """ceil(tokens / experts * capacity_factor), at least min_capacity (topk_gating.py:13-22; the product is
     formed with an fp32 tensor there, reproduced here so the integer agrees)."""
-    cap = torch.ceil((num_tokens / num_experts) * torch.tensor(capacity_factor)).to(torch.int64)
+    cap = math.ceil(_f32(_f32(num_tokens / num_experts) * _f32(capacity_factor)))
     return max(int(cap), int(min_capacity))
 
 
@@ -36,7 +43,7 @@ class TopKGatingFunc(torch.autograd.Function):
         ec_idx = torch.empty(k * S, dtype=torch.int32, device=dev)
         weights = torch.empty(k * S, dtype=torch.float32, device=dev)
         select = torch.empty(E * capacity, dtype=torch.int64, device=dev)
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             _lib.check(lib.dlb_gshard_forward(x.data_ptr(), S, E, k, capacity, gates.data_ptr(), ids_km.data_ptr(),
                                               colsum.data_ptr(), colsum.numel(), loc.data_ptr(), me.data_ptr(),
                                               ce.data_ptr(), l_aux.data_ptr(), ec_idx.data_ptr(), weights.data_ptr(),
@@ -60,7 +67,7 @@ class TopKGatingFunc(torch.autograd.Function):
         g = (torch.zeros(1, device=dev) if grad_l_aux is None else grad_l_aux.float().reshape(1)).contiguous()
         grad_logits = torch.empty_like(gates)
         lib = _lib.load()
-        with torch.cuda.device(dev):
+        with _lib.on_device(dev):
             if ctx.higher_precision:
                 # the routing weights back-propagate too (topk_gating.py:286-294).  The gradient is the exact
                 # derivative of weights = kept gate / max(sum of kept gates, eps); the reference's kernel divides
