@@ -73,6 +73,8 @@ SIGNATURES = {
                                  c_int64, c_int64, c_int64, c_int64, c_int64, c_int64,
                                  c_int64, c_int, c_int, c_int64, c_int64, c_int64, c_float, c_float, c_int,
                                  c_void_p, c_void_p]),
+    "dlb_paged_decode_rows": (c_int, [c_void_p] * 6 + [c_int64, c_int] + [c_void_p] * 2 + [c_int64] * 19 +
+                              [c_int, c_int, c_int64, c_int64, c_int64, c_float, c_float, c_int, c_void_p, c_void_p]),
     "dlb_rms_norm": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                              c_int64, c_float, c_int, c_int, c_void_p]),
     "dlb_apply_rotary": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int,

@@ -89,6 +89,8 @@ struct DecodeParams {
   int64_t q_stride_b, q_stride_h;
   int64_t o_stride_b, o_stride_h;
   int64_t bt_stride;
+  const void* table_rows;    // [B] row of the block table of every sequence (int32 or int64), or null: row b
+  int num_table_rows, rows_is_int64;
   int batch, hq, hkv, group;
   int dk, dv;                // true head sizes of q/k and of v/out (<= D, multiples of 8); columns beyond them are zero
   int page_size, max_pages, num_pages;
@@ -177,6 +179,9 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
     return;   // whole CTA leaves
   }
   const int n_tiles = (hi - lo + TILE_KEYS - 1) / TILE_KEYS;
+  int64_t table_row = b;
+  if (p.table_rows != nullptr)
+    table_row = min(max(load_index(p.table_rows, b, p.rows_is_int64), 0), p.num_table_rows - 1);
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -244,7 +249,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         const int tok = lo + t * TILE_KEYS + q * GATHER_ROWS + (lane % GATHER_ROWS);
         int page_slot = one_token_pages ? tok : (tok >> p.page_shift);
         if (page_slot >= p.max_pages) page_slot = p.max_pages - 1;   // rows past the table: any valid page
-        int page = load_index(p.block_table, (int64_t)b * p.bt_stride + page_slot, p.table_is_int64);
+        int page = load_index(p.block_table, table_row * p.bt_stride + page_slot, p.table_is_int64);
         if (tok >= ctx || page < 0 || page >= p.num_pages) page = 0;  // masked later; keep the address legal
         pg = page;
         sl = tok & (p.page_size - 1);
@@ -300,7 +305,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         const int tok = tok0 + bx * keys_per_box;
         int page_slot = tok / p.page_size;
         if (page_slot >= p.max_pages) page_slot = p.max_pages - 1;   // tail boxes past the table: any valid page
-        int page = load_index(p.block_table, (int64_t)b * p.bt_stride + page_slot, p.table_is_int64);
+        int page = load_index(p.block_table, table_row * p.bt_stride + page_slot, p.table_is_int64);
         if (tok >= ctx || page < 0 || page >= p.num_pages) page = 0;  // masked later; keep the address legal
         const int slot0 = tok % p.page_size;
 #pragma unroll
@@ -573,18 +578,21 @@ extern "C" int64_t dlb_paged_decode_workspace_floats(int64_t batch, int64_t hq, 
   return max_splits <= 1 ? 0 : batch * hq * max_splits * (width + 2);
 }
 
-extern "C" int dlb_paged_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
-                                const void* block_table, const void* kv_seqlens, float* partial, int64_t batch,
-                                int64_t hq, int64_t hkv, int64_t head_dim, int64_t head_dim_v, int64_t page_size,
-                                int64_t num_pages, int64_t max_pages, int64_t q_stride_b, int64_t q_stride_h,
-                                int64_t o_stride_b,
-                                int64_t o_stride_h, int64_t k_stride_page, int64_t k_stride_slot,
-                                int64_t k_stride_head, int64_t v_stride_page, int64_t v_stride_slot,
-                                int64_t v_stride_head, int64_t bt_stride, int table_is_int64, int lens_is_int64,
-                                int64_t chunk, int64_t max_splits, int64_t window, float sm_scale, float softcap,
-                                int dtype, int32_t* status, void* stream) {
+extern "C" int dlb_paged_decode_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                     const void* block_table, const void* table_rows, int64_t num_table_rows,
+                                     int rows_is_int64, const void* kv_seqlens, float* partial, int64_t batch,
+                                     int64_t hq, int64_t hkv, int64_t head_dim, int64_t head_dim_v, int64_t page_size,
+                                     int64_t num_pages, int64_t max_pages, int64_t q_stride_b, int64_t q_stride_h,
+                                     int64_t o_stride_b, int64_t o_stride_h, int64_t k_stride_page,
+                                     int64_t k_stride_slot, int64_t k_stride_head, int64_t v_stride_page,
+                                     int64_t v_stride_slot, int64_t v_stride_head, int64_t bt_stride,
+                                     int table_is_int64, int lens_is_int64, int64_t chunk, int64_t max_splits,
+                                     int64_t window, float sm_scale, float softcap, int dtype, int32_t* status,
+                                     void* stream) {
   DLB_NVTX("dlb_paged_decode");
   using namespace dlb;
+  DLB_CHECK_ARG(table_rows == nullptr || (num_table_rows >= 1 && num_table_rows < (1LL << 31)), DLB_ERR_BAD_ARG,
+                "paged_decode: table of %lld rows", (long long)num_table_rows);
   DLB_CHECK_ARG(dtype == DLB_DTYPE_BF16 || dtype == DLB_DTYPE_F16, DLB_ERR_UNSUPPORTED,
                 "paged_decode: dtype %d (need fp16 or bf16)", dtype);
   DLB_CHECK_ARG(head_dim >= 8 && head_dim <= 128 && head_dim % 8 == 0 && head_dim_v >= 8 && head_dim_v <= 128 &&
@@ -627,6 +635,9 @@ extern "C" int dlb_paged_decode(const void* q, const void* k_cache, const void* 
   p.o_stride_b = o_stride_b;
   p.o_stride_h = o_stride_h;
   p.bt_stride = bt_stride;
+  p.table_rows = table_rows;
+  p.num_table_rows = (int)num_table_rows;
+  p.rows_is_int64 = rows_is_int64;
   p.batch = (int)batch;
   p.hq = (int)hq;
   p.hkv = (int)hkv;
@@ -669,6 +680,23 @@ extern "C" int dlb_paged_decode(const void* q, const void* k_cache, const void* 
                         : launch_decode<__nv_bfloat16, 64>(tk, tv, p, s);
   }
   return width == 128 ? launch_decode<__half, 128>(tk, tv, p, s) : launch_decode<__half, 64>(tk, tv, p, s);
+}
+
+extern "C" int dlb_paged_decode(const void* q, const void* k_cache, const void* v_cache, void* out,
+                                const void* block_table, const void* kv_seqlens, float* partial, int64_t batch,
+                                int64_t hq, int64_t hkv, int64_t head_dim, int64_t head_dim_v, int64_t page_size,
+                                int64_t num_pages, int64_t max_pages, int64_t q_stride_b, int64_t q_stride_h,
+                                int64_t o_stride_b,
+                                int64_t o_stride_h, int64_t k_stride_page, int64_t k_stride_slot,
+                                int64_t k_stride_head, int64_t v_stride_page, int64_t v_stride_slot,
+                                int64_t v_stride_head, int64_t bt_stride, int table_is_int64, int lens_is_int64,
+                                int64_t chunk, int64_t max_splits, int64_t window, float sm_scale, float softcap,
+                                int dtype, int32_t* status, void* stream) {
+  return dlb_paged_decode_rows(q, k_cache, v_cache, out, block_table, nullptr, 0, 0, kv_seqlens, partial, batch, hq,
+                               hkv, head_dim, head_dim_v, page_size, num_pages, max_pages, q_stride_b, q_stride_h,
+                               o_stride_b, o_stride_h, k_stride_page, k_stride_slot, k_stride_head, v_stride_page,
+                               v_stride_slot, v_stride_head, bt_stride, table_is_int64, lens_is_int64, chunk,
+                               max_splits, window, sm_scale, softcap, dtype, status, stream);
 }
 
 // ----------------------------------------------------------------------------

@@ -37,23 +37,27 @@ def decode_attention_fwd(
     assert D % 8 == 0 and Dv % 8 == 0 and D <= 128 and Dv <= 128, "head sizes: multiples of 8 up to 128"
     assert q.stride(-1) == 1 and o.stride(-1) == 1 and k_buffer.stride(-1) == 1 and v_buffer.stride(-1) == 1
     hkv = k_buffer.shape[1]
-    table = req_to_token.index_select(0, b_req_idx.to(torch.int64))
-    if table.dtype not in (torch.int32, torch.int64):
-        table = table.to(torch.int64)
-    max_ctx = min(int(max_len_in_batch), table.size(1)) if max_len_in_batch else table.size(1)
-    table = table[:, :max(max_ctx, 1)].contiguous()
+    # the kernel looks its row up itself: gathering the rows of 16 requests of up to 32768 tokens first took 17 us of 234
+    table = req_to_token if req_to_token.dtype in (torch.int32, torch.int64) else req_to_token.to(torch.int64)
+    if table.stride(1) != 1:
+        table = table.contiguous()
+    rows = b_req_idx if b_req_idx.dtype in (torch.int32, torch.int64) else b_req_idx.to(torch.int64)
+    rows = rows.reshape(-1).contiguous()
+    assert rows.size(0) >= batch, "b_req_idx: one table row per request"
+    max_ctx = max(min(int(max_len_in_batch), table.size(1)) if max_len_in_batch else table.size(1), 1)
     lens = b_seq_len if b_seq_len.dtype in (torch.int32, torch.int64) else b_seq_len.to(torch.int64)
     lens = lens.contiguous()
-    chunk = _pick_chunk(batch, hkv, table.size(1), 1)
-    max_splits = (table.size(1) + chunk - 1) // chunk
+    chunk = _pick_chunk(batch, hkv, max_ctx, 1)
+    max_splits = (max_ctx + chunk - 1) // chunk
     lib = _lib.load()
     nfloats = lib.dlb_paged_decode_workspace_floats(batch, head, max(D, Dv), max_splits)
     partial = torch.empty(max(nfloats, 1), dtype=torch.float32, device=dev)
     status = _lib.status_word(dev)
     with _lib.on_device(dev):
-        rc = lib.dlb_paged_decode(
-            q.data_ptr(), k_buffer.data_ptr(), v_buffer.data_ptr(), o.data_ptr(), table.data_ptr(), lens.data_ptr(),
-            partial.data_ptr(), batch, head, hkv, D, Dv, 1, k_buffer.size(0), table.size(1),
+        rc = lib.dlb_paged_decode_rows(
+            q.data_ptr(), k_buffer.data_ptr(), v_buffer.data_ptr(), o.data_ptr(), table.data_ptr(), rows.data_ptr(),
+            table.size(0), int(rows.dtype == torch.int64), lens.data_ptr(),
+            partial.data_ptr(), batch, head, hkv, D, Dv, 1, k_buffer.size(0), max_ctx,
             q.stride(0), q.stride(1), o.stride(0), o.stride(1),
             k_buffer.stride(0), k_buffer.stride(0), k_buffer.stride(1),
             v_buffer.stride(0), v_buffer.stride(0), v_buffer.stride(1),

@@ -266,6 +266,18 @@ int dlb_paged_decode(const void* q, const void* k_cache, const void* v_cache, vo
                      int lens_is_int64, int64_t chunk, int64_t max_splits, int64_t window, float sm_scale,
                      float softcap, int dtype, int32_t* status, void* stream);
 
+/* The same with one more indirection: sequence b reads row table_rows[b] (int32 or int64, clamped to
+ * [0, num_table_rows)) of block_table instead of row b; table_rows == NULL is dlb_paged_decode. */
+int dlb_paged_decode_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
+                          const void* block_table, const void* table_rows, int64_t num_table_rows,
+                          int rows_is_int64, const void* kv_seqlens, float* partial, int64_t batch, int64_t hq,
+                          int64_t hkv, int64_t head_dim, int64_t head_dim_v, int64_t page_size, int64_t num_pages,
+                          int64_t max_pages, int64_t q_stride_b, int64_t q_stride_h, int64_t o_stride_b,
+                          int64_t o_stride_h, int64_t k_stride_page, int64_t k_stride_slot, int64_t k_stride_head,
+                          int64_t v_stride_page, int64_t v_stride_slot, int64_t v_stride_head, int64_t bt_stride,
+                          int table_is_int64, int lens_is_int64, int64_t chunk, int64_t max_splits, int64_t window,
+                          float sm_scale, float softcap, int dtype, int32_t* status, void* stream);
+
 /* rms_norm with optional residual add.  new_x = x + residual in the storage dtype (written to
  * out_residual when given); out = w * (new_x * rsqrt(mean(new_x^2) + eps)).  weight_after_cast = 0
  * multiplies in fp32 and rounds once (python/dlBLAS/dlblas/kernels/rms_norm.py:8-132);
