@@ -105,15 +105,19 @@ template <typename T> __device__ __forceinline__ float round_to(float a) { retur
 // of the range, kept the 32 elements of a step from overlapping: the epilogue of a tile took about 55 000 clocks, and
 // every gate/up launch with a shorter main loop waited for it (32 experts, K = 1024: 235 us for 369 MB of weights).
 // Whole fused_moe, before -> after: 2000 tokens over 256 experts (2048 x 1024) 676 -> 600 us, 128 over 64 (2048 x 1408)
-// 246 -> 203, 32 over 32 (1024 x 2816) 195 -> 113, 4096 over 8 (4096 x 14336) 2394 -> 2298; same outputs bit for bit.
-// Both sides are scaled by 1/4 so that the reciprocal of the largest 1 + e^-x is not subnormal.
+// 246 -> 203, 32 over 32 (1024 x 2816) 195 -> 113, 4096 over 8 (4096 x 14336) 2394 -> 2298.
+// Both sides are scaled by 1/4 so that the reciprocal of the largest 1 + e^-x is not subnormal.  Where e^-x is infinite
+// (x below -88.7) the quotient is -0, or NaN at -inf; at +inf the correction would make it NaN.  Rounded to the type,
+// every 16-bit x gives what the division gives.
 __device__ __forceinline__ float silu_branchless(float x) {
-  const float d = fmaf(fminf(__expf(-x), 3.402823466e38f), 0.25f, 0.25f), a = x * 0.25f;
+  const float e = __expf(-x);
+  const float d = fmaf(e, 0.25f, 0.25f), a = x * 0.25f;
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
   const float q = a * r;
   const float s = fmaf(fmaf(-q, d, a), r, q);
-  return x > 3.402823466e38f ? x : s;      // +inf; the correction would make it NaN (as the division does for -inf)
+  const float low = e > 3.402823466e38f ? x * 0.f : s;
+  return x > 3.402823466e38f ? x : low;
 }
 
 // silu(gate) * up with the reference's rounding points.

@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from dlcompiler_b200 import fused_moe
+from dlcompiler_b200 import _lib, fused_moe
+from dlcompiler_b200.kernels.fused_moe import _grouped_gemm
 from oracle import dlblas_oracle as oracle
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +48,33 @@ def test_silu_over_its_range(cuda_device, dtype):
                     torch.eye(n).unsqueeze(0).to(dtype).to(cuda_device), one, one.long() * 0, 1)
     ref = torch.nn.functional.silu(values.double())
     torch.testing.assert_close(out[0].cpu().double(), ref, rtol=2 * torch.finfo(dtype).eps, atol=2.0 ** -24)
+
+
+@pytest.mark.parametrize("few", [True, False])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_silu_of_every_value(cuda_device, dtype, few):
+    """The activation of all 65536 gates of the type, straight from the GEMM that fuses it, up = 1.  Where e^-x leaves
+    fp32 (x < -88.73) the quotient is -0, whatever the size of x, and NaN at -inf; elsewhere two roundings to the type and
+    the relative error of exp's fp32 argument (|x| 2^-24, below 2^-17)."""
+    gates = torch.arange(-32768, 32768, dtype=torch.int32).to(torch.int16).view(dtype)
+    n = gates.numel()
+    w1 = torch.zeros(1, 2 * n, 8, dtype=dtype)
+    w1[0, :n, 0], w1[0, n:, 0] = gates, 1.0
+    a = torch.zeros(128, 8, dtype=dtype)
+    a[0, 0] = 1.0
+    numel = 1 if few else 128            # the padding's share picks the kernel's form
+    ids = torch.full((128,), numel, dtype=torch.int32)
+    ids[0] = 0
+    out = torch.zeros(128, n, dtype=dtype, device=cuda_device)
+    _grouped_gemm(a.to(cuda_device), w1.to(cuda_device), out, n, ids.to(cuda_device),
+                  torch.tensor([0, 1], dtype=torch.int32, device=cuda_device), None, numel, _lib.GEMM_FUSE_SILU)
+    got, x = out[0].cpu().double(), gates.double()
+    ref = torch.nn.functional.silu(x)
+    gone = x < -88.73
+    assert torch.equal(got[gone & torch.isfinite(x)], ref.new_zeros(int((gone & torch.isfinite(x)).sum())))
+    assert torch.isnan(got[x == -torch.inf]).all() and torch.isnan(got[torch.isnan(x)]).all()
+    assert (got[x == torch.inf] == torch.inf).all()
+    rest = torch.isfinite(x) & ~gone
+    # the smallest normal number as the floor: the tensor cores may take a subnormal operand as zero
+    torch.testing.assert_close(got[rest], ref[rest], rtol=2 * torch.finfo(dtype).eps + 2.0 ** -17,
+                               atol=torch.finfo(dtype).tiny)
