@@ -16,6 +16,7 @@ LIB_PATH = os.path.join(_PKG_DIR, "libdlblas_b200.so")
 
 DTYPE_F16, DTYPE_BF16, DTYPE_F32 = 0, 1, 2
 SCORE_SIGMOID, SCORE_SOFTMAX = 0, 1
+DEV_BAD_ROW = 2  # code in a device status word
 GEMM_FUSE_SILU, GEMM_WEIGHT, GEMM_SCATTER, GEMM_PEER = 1, 2, 4, 8
 
 _DTYPES = {torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16, torch.float32: DTYPE_F32}
@@ -185,7 +186,7 @@ _status_words: dict[int, torch.Tensor] = {}
 
 
 def status_word(device: torch.device) -> torch.Tensor:
-    """Per-device int32[4] the tensor-core kernels write when a bounded wait gives up."""
+    """Per-device int32[4] that a kernel writes when a bounded wait gives up or a table row does not exist."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
     t = _status_words.get(idx)
     if t is None:
@@ -207,7 +208,7 @@ def set_wait_budget_ms(ms: int) -> None:
 
 
 def check_device_status(device=None) -> None:
-    """Synchronise and raise if any kernel recorded a timed-out wait since the last check."""
+    """Synchronise and raise if any kernel recorded a timed-out wait or a bad table row since the last check."""
     devs = list(_status_words) if device is None else [torch.device(device).index or 0]
     for idx in devs:
         t = _status_words.get(idx)
@@ -216,5 +217,8 @@ def check_device_status(device=None) -> None:
         vals = t.cpu().tolist()
         if vals[0] != 0:
             t.zero_()
+            if vals[0] == DEV_BAD_ROW:
+                raise DlblasError(f"device status on cuda:{idx}: request {vals[1]} of a decode asked for row {vals[3]} "
+                                  f"of a table of {vals[2]}")
             raise DlblasError(
                 f"device status on cuda:{idx}: code={vals[0]} wait_site={vals[1]} block={vals[2]} aux={vals[3]}")

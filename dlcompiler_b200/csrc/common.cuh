@@ -45,11 +45,13 @@ struct NvtxRange {
 // (DLB_DTYPE_*) and the flag values of the boundary come from there.
 #include "dlblas_b200.h"
 
-// Layout of the device status word array (int32[4]) that kernels with bounded
-// waits write when they give up:  [0] = error code (0 = none), [1] = wait site,
-// [2] = blockIdx.x, [3] = auxiliary value (tile / iteration).
+// Layout of the device status word array (int32[4]), written by the first kernel that has something to report:
+// [0] = code (0 = none).  A bounded wait that gave up: [1] = wait site, [2] = blockIdx.x, [3] = auxiliary value
+// (tile / iteration).  A table row that does not exist: [1] = sequence, [2] = rows of the table, [3] = the row asked for
+// (clamped to 32 bits).
 #define DLB_DEV_OK 0
 #define DLB_DEV_WAIT_TIMEOUT 1
+#define DLB_DEV_BAD_ROW 2
 
 namespace dlb {
 

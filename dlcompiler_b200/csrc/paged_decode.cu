@@ -128,6 +128,12 @@ __device__ __forceinline__ int load_index(const void* p, int64_t i, int is64) {
   return is64 ? (int)reinterpret_cast<const int64_t*>(p)[i] : reinterpret_cast<const int32_t*>(p)[i];
 }
 
+// Row of the block table that sequence b reads, as it stands in table_rows (64 bits: not cut before it is compared).
+__device__ __forceinline__ int64_t named_row(const DecodeParams& p, int b) {
+  return p.rows_is_int64 ? reinterpret_cast<const int64_t*>(p.table_rows)[b]
+                         : reinterpret_cast<const int32_t*>(p.table_rows)[b];
+}
+
 // Token range [lo, hi) of split `s`; returns false if the split is empty.
 __device__ __forceinline__ bool split_range(int ctx, int window, int chunk, int s, int& lo, int& hi, int& kv_lo) {
   // the query sits at position ctx - 1 and sees keys ctx - 1 - window .. ctx - 1, as in the reference
@@ -167,7 +173,21 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  const int ctx = load_index(p.kv_seqlens, b, p.lens_is_int64);
+  int ctx = load_index(p.kv_seqlens, b, p.lens_is_int64);
+  int64_t table_row = b;
+  if constexpr (ROWS) {
+    // a row outside the table names nobody's tokens: the sequence counts as empty and the call is recorded as wrong
+    table_row = named_row(p, b);
+    if (table_row < 0 || table_row >= p.num_table_rows) {
+      ctx = 0;
+      if (split == 0 && blockIdx.y == 0 && threadIdx.x == 0 && p.status != nullptr &&
+          atomicCAS(p.status, DLB_DEV_OK, DLB_DEV_BAD_ROW) == DLB_DEV_OK) {
+        p.status[1] = b;
+        p.status[2] = p.num_table_rows;
+        p.status[3] = (int)max((int64_t)INT32_MIN, min(table_row, (int64_t)INT32_MAX));
+      }
+    }
+  }
   int lo, hi, kv_lo;
   if (!split_range(ctx, p.window, p.chunk, split, lo, hi, kv_lo)) {
     // empty split: nothing to do, except that without a merge pass an empty context still owes zeros
@@ -206,8 +226,6 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 
   if (warp >= CONSUMER_WARPS) {
     // ------------------------------ producer ------------------------------
-    int64_t table_row = b;
-    if constexpr (ROWS) table_row = min(max(load_index(p.table_rows, b, p.rows_is_int64), 0), p.num_table_rows - 1);
     // A tile is 64 keys = 64 / min(page, 64) boxes per K/V half; the boxes are spread over the
     // lanes of this warp so that small pages (down to one token per page) still issue quickly.
     if (lane == 0) {
@@ -526,7 +544,11 @@ __global__ void __launch_bounds__(D) paged_decode_merge_kernel(const DecodeParam
   const int head = blockIdx.x;
   const int b = blockIdx.y;
   const int d = threadIdx.x;
-  const int ctx = load_index(p.kv_seqlens, b, p.lens_is_int64);
+  int ctx = load_index(p.kv_seqlens, b, p.lens_is_int64);
+  if (p.table_rows != nullptr) {
+    const int64_t row = named_row(p, b);
+    if (row < 0 || row >= p.num_table_rows) ctx = 0;      // as the split kernel has it
+  }
   T* out = reinterpret_cast<T*>(p.out) + (int64_t)b * p.o_stride_b + (int64_t)head * p.o_stride_h;
   int lo, hi, kv_lo;
   if (!split_range(ctx, p.window, p.chunk, 0, lo, hi, kv_lo)) {

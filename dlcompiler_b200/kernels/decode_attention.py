@@ -28,6 +28,8 @@ def decode_attention_fwd(
     (decode_attention.py:559-620); here the same math is one split-KV pass of the paged decode
     kernel with a page size of one token, so `attn_logits` and `b_start_loc` are accepted for
     signature compatibility and not touched.  `logit_cap > 0` applies cap * tanh(qk / cap).
+
+    A `b_req_idx[i]` outside `req_to_token` is an error: the request gets zeros and `check_device_status()` raises.
     """
     dev = _lib.require_cuda(q, k_buffer, v_buffer, o, req_to_token, b_req_idx, b_seq_len)
     assert q.dim() == 3 and k_buffer.dim() == 3 and v_buffer.dim() == 3

@@ -10,7 +10,8 @@
  *     > 0 a cudaError_t from the launch;
  *   - `status` (optional, may be NULL) is a device int32[4] the tensor-core kernels
  *     write if one of their bounded waits gives up:
- *     {code (0 = none, 1 = wait timed out), wait site, block index, tile}.
+ *     {code (0 = none, 1 = wait timed out), wait site, block index, tile}
+ *     (dlb_paged_decode_rows has a code 2 of its own).
  *
  * Paths below are relative to the reference project root (DeepLink-org/DLCompiler).
  */
@@ -266,8 +267,9 @@ int dlb_paged_decode(const void* q, const void* k_cache, const void* v_cache, vo
                      int lens_is_int64, int64_t chunk, int64_t max_splits, int64_t window, float sm_scale,
                      float softcap, int dtype, int32_t* status, void* stream);
 
-/* The same with one more indirection: sequence b reads row table_rows[b] (int32 or int64, clamped to
- * [0, num_table_rows)) of block_table instead of row b; table_rows == NULL is dlb_paged_decode. */
+/* The same with one more indirection: sequence b reads row table_rows[b] (int32 or int64) of block_table instead of
+ * row b; table_rows == NULL is dlb_paged_decode.  A row outside [0, num_table_rows) reads nothing: its sequence gets
+ * zeros and `status` the code 2 with {sequence, num_table_rows, the row}. */
 int dlb_paged_decode_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
                           const void* block_table, const void* table_rows, int64_t num_table_rows,
                           int rows_is_int64, const void* kv_seqlens, float* partial, int64_t batch, int64_t hq,

@@ -2,7 +2,8 @@
 import pytest
 import torch
 
-from dlcompiler_b200 import decode_attention_fwd
+from dlcompiler_b200 import check_device_status, decode_attention_fwd
+from dlcompiler_b200._lib import DlblasError
 
 pytestmark = pytest.mark.gpu
 
@@ -24,3 +25,28 @@ def test_rows_of_the_table(cuda_device, idx_dtype, transposed):
     decode_attention_fwd(q, k, v, ref, pool[idx.to(cuda_device)].contiguous(), torch.arange(5, device=cuda_device), None,
                          lens, None, ctx, 0.125)
     assert torch.isfinite(out.float()).all() and torch.equal(out, ref)
+
+
+@pytest.mark.parametrize("ctx", [64, 4000])             # one split, and the merge of several
+@pytest.mark.parametrize("bad,idx_dtype", [(-1, torch.int32), (7, torch.int32), (-1, torch.int64), (7, torch.int64),
+                                           (2 ** 32 + 3, torch.int64), (-2 ** 40, torch.int64)])
+def test_row_outside_the_table(cuda_device, bad, idx_dtype, ctx):
+    """No other request's tokens: zeros for that request, an error for the call, the other requests as without it."""
+    g = torch.Generator().manual_seed(5)
+    rows, hq, hkv, dim = 7, 8, 2, 64
+    pool = torch.randint(0, 5000, (rows, ctx), generator=g, dtype=torch.int32).to(cuda_device)
+    k, v = (torch.randn(5000, hkv, dim, generator=g).to(torch.bfloat16).to(cuda_device) for _ in range(2))
+    q = torch.randn(3, hq, dim, generator=g).to(torch.bfloat16).to(cuda_device)
+    lens = torch.tensor([ctx, ctx - 1, ctx // 2], dtype=torch.int32, device=cuda_device)
+    outs = []
+    for idx in ([6, 3, 0], [6, bad, 0]):
+        o = torch.full_like(q, 7.0)
+        decode_attention_fwd(q, k, v, o, pool, torch.tensor(idx, dtype=idx_dtype, device=cuda_device), None, lens, None,
+                             ctx, 0.125)
+        outs.append(o)
+        if bad in idx:
+            with pytest.raises(DlblasError, match="request 1 .* table of 7"):
+                check_device_status()
+        check_device_status()
+    assert torch.equal(outs[1][1], torch.zeros_like(q[1]))
+    assert torch.equal(outs[1][[0, 2]], outs[0][[0, 2]])
