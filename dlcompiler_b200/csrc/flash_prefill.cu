@@ -181,10 +181,9 @@ __device__ __forceinline__ int table_entry(const void* t, int64_t i, int is64) {
 //                     light ones; for K/V that stay in L2 altogether.
 //   ORDER_RAGGED      ORDER_TILES over the tiles that exist, the CTAs without work last: on 13 prompts of 17 to 901
 //                     tokens half the CTAs of the full grid have none, and spread over it they cost 13 us of 95.
-// The sorted forms keep one sequence per lane (batch <= 32).  Measured on B200, 32 / 8 heads of 128, causal, together
-// with the early first loads and the staged epilogue, before -> after: 1 x 2048 tokens 58 -> 47 us, 1 x 8192 512 -> 470,
-// 8 x 2048 328 -> 303, 8 x 256 20.2 -> 18.6, the 13 prompts 95 -> 88; four chunks of 256-768 tokens over 1000-8000
-// cached ones 249 -> 235.  16 x 64 tokens, all in flight at once, 12.3 -> 12.9.
+// The sorted forms keep one sequence per lane (batch <= 32).  Measured on B200, 32 / 8 heads of 128, causal, cold L2, with
+// the early first loads and the epilogue below, ORDER_GROUPS for all with neither -> now: 1 x 2048 tokens 67.9 -> 55.1 us,
+// 1 x 8192 522 -> 472, 8 x 2048 346 -> 313, 64 x 256 135.0 -> 127.4, 64 x 64 46.8 -> 45.4, 13 prompts 88.8 -> 84.3.
 __device__ __forceinline__ bool prefill_tile(const PrefillParams& p, int x, int& seq, int& tile, int& head) {
   if (p.order == fp::ORDER_GROUPS) {
     const int hig = x % p.group;
@@ -623,38 +622,64 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       tc_fence_after_sync();
       const float inv_l = 1.f / l_sum;
       const bool row_ok = q_pos < seq_len;
-      // Through the Q tile's shared memory (every Q K^T has retired; row r of O over row r of Q, same swizzle), so that
-      // the lanes of a store cover whole rows instead of 16 bytes of 32 rows each.
-      uint8_t* stage = smem + OFF_Q;
-      const int rows = min(32, seq_len - q0 - quad * 32);   // the warp's rows inside the sequence
-#pragma unroll 1
-      for (int c = 0; rows > 0 && c < D / 64; ++c) {
-        uint32_t o[2][32];
-        tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64, o[0]);
-        tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64 + 32, o[1]);
-        tmem_wait_ld();
+      auto pack_row = [](const uint32_t* acc, float scale) {     // eight accumulators as one 16-byte chunk
+        uint32_t w[4];
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          uint32_t w[4];
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t* pair = &o[v >> 2][(v & 3) * 8 + 2 * i];
-            typename Elem<T>::T2 v2 = Elem<T>::from_f2(__uint_as_float(pair[0]) * inv_l, __uint_as_float(pair[1]) * inv_l);
-            w[i] = *reinterpret_cast<uint32_t*>(&v2);
-          }
-          *reinterpret_cast<uint4*>(stage + c * Q_BOX + row * 128 + ((v ^ (row & 7)) << 4)) =
-              make_uint4(w[0], w[1], w[2], w[3]);
+        for (int i = 0; i < 4; ++i) {
+          typename Elem<T>::T2 v2 = Elem<T>::from_f2(__uint_as_float(acc[2 * i]) * scale, __uint_as_float(acc[2 * i + 1]) * scale);
+          w[i] = *reinterpret_cast<uint32_t*>(&v2);
         }
-      }
-      __syncwarp();
-      constexpr int LANES = D / 8;       // lanes per row
-      const int cc = lane % LANES;       // 16-byte chunk of the row
-      T* obase = reinterpret_cast<T*>(p.out) + (int64_t)head * p.o_stride_h + cc * 8;
-#pragma unroll 4
-      for (int i = lane / LANES; i < rows; i += 32 / LANES) {
-        const int r = quad * 32 + i;
-        const uint4 val = *reinterpret_cast<const uint4*>(stage + (cc >> 3) * Q_BOX + r * 128 + (((cc & 7) ^ (r & 7)) << 4));
-        if (cc * 8 < p.dv) *reinterpret_cast<uint4*>(obase + (int64_t)(start + q0 + r) * p.o_stride_t) = val;
+        return make_uint4(w[0], w[1], w[2], w[3]);
+      };
+      if (seq_len - q0 <= 64) {
+        // Few rows: each lane stores its own.  With at most two warps that have rows there is little to hide the way
+        // through shared memory behind (64 x 64 tokens: 50.3 us staged, 45.4 so; 128 x 40: 91.2, 80.7).
+        T* orow = reinterpret_cast<T*>(p.out) + (int64_t)(start + q_pos) * p.o_stride_t + (int64_t)head * p.o_stride_h;
+#pragma unroll 1
+        for (int c = 0; c < D / 32; ++c) {
+          uint32_t o[32];
+          tmem_ld_32x32b_x32(tmem_o + lane_field + c * 32, o);
+          tmem_wait_ld();
+          if (row_ok) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              const uint4 w = pack_row(o + v * 8, inv_l);
+              if (c * 32 + v * 8 < p.dv) *reinterpret_cast<uint4*>(orow + c * 32 + v * 8) = w;
+            }
+          }
+        }
+      } else {
+        // Through the Q tile's shared memory (every Q K^T has retired; row r of O over row r of Q, same swizzle), 64
+        // columns at a time, so that the lanes of a store cover whole 128-byte lines instead of 16 bytes of 32 rows each
+        // (8 x 2048 tokens: 324.9 us with a row per lane, 313.1 so; 64 x 256: 135.4, 127.4).
+        uint8_t* stage = smem + OFF_Q;
+        const int rows = min(32, seq_len - q0 - quad * 32);   // the warp's rows inside the sequence
+        const int sub = lane >> 3, cc = lane & 7;              // row of four, 16-byte chunk of its line
+        T* obase = reinterpret_cast<T*>(p.out) + (int64_t)(start + q0 + quad * 32 + sub) * p.o_stride_t +
+                   (int64_t)head * p.o_stride_h + cc * 8;
+#pragma unroll 1
+        for (int c = 0; rows > 0 && c < D / 64; ++c) {
+          uint32_t o[2][32];
+          tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64, o[0]);
+          tmem_ld_32x32b_x32(tmem_o + lane_field + c * 64 + 32, o[1]);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            *reinterpret_cast<uint4*>(stage + c * Q_BOX + row * 128 + ((v ^ (row & 7)) << 4)) =
+                pack_row(o[v >> 2] + (v & 3) * 8, inv_l);
+          __syncwarp();
+          uint4 val[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const int r = quad * 32 + i * 4 + sub;
+            val[i] = *reinterpret_cast<const uint4*>(stage + c * Q_BOX + r * 128 + ((cc ^ (r & 7)) << 4));
+          }
+          if (c * 64 + cc * 8 < p.dv) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+              if (i * 4 + sub < rows) *reinterpret_cast<uint4*>(obase + (int64_t)(i * 4) * p.o_stride_t + c * 64) = val[i];
+          }
+        }
       }
       if (row_ok && p.lse != nullptr) {
         p.lse[(int64_t)head * p.total_tokens + start + q_pos] = m_ref * 0.6931471805599453f + __logf(l_sum);

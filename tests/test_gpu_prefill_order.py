@@ -36,6 +36,21 @@ def test_varlen_orders(cuda_device, lens, dim):
     torch.testing.assert_close(lse.cpu(), rlse, rtol=1e-3, atol=1e-3)
 
 
+@pytest.mark.parametrize("dim", [128, 64, 72, 24])
+@pytest.mark.parametrize("rows", [1, 32, 33, 63, 64, 65, 96, 97, 127, 128, 129, 192, 193])
+def test_epilogue_by_rows_of_the_tile(cuda_device, rows, dim):
+    """Both ways out of a tile at their edges (at most 64 rows: a row per lane; more: staged), into a strided output
+    whose other columns and rows stay as they are."""
+    q, k, v, start, n = _case([rows], 4, 2, dim, rows)
+    wide = torch.full((rows + 3, 4, dim + 8), 7.0, dtype=torch.bfloat16, device=cuda_device)
+    o = wide[:rows, :, :dim]
+    context_attention_fwd(q.to(cuda_device), k.to(cuda_device), v.to(cuda_device), o, start.to(cuda_device),
+                          n.to(cuda_device), rows)
+    ref = oracle.context_attention(q, k, v, start, n)
+    torch.testing.assert_close(o.cpu().float(), ref.float(), rtol=RTOL, atol=ATOL)
+    assert (wide[rows:] == 7).all() and (wide[:, :, dim:] == 7).all()
+
+
 @pytest.mark.parametrize("batch", [5, 32, 33])
 def test_paged_sequences_by_length(cuda_device, batch):
     """More tiles than the GPU holds at once: sequences by descending key count, up to 32 of them.  A sequence
