@@ -91,6 +91,7 @@ struct DecodeParams {
   int64_t bt_stride;
   const void* table_rows;    // [B] row of the block table of every sequence (int32 or int64), or null: row b
   int num_table_rows, rows_is_int64;
+  int rows_gathered;         // the table holds the named rows in the order of the batch: row b, if the named one exists
   int batch, hq, hkv, group;
   int dk, dv;                // true head sizes of q/k and of v/out (<= D, multiples of 8); columns beyond them are zero
   int page_size, max_pages, num_pages;
@@ -187,6 +188,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         p.status[3] = (int)max((int64_t)INT32_MIN, min(table_row, (int64_t)INT32_MAX));
       }
     }
+    if (p.rows_gathered) table_row = b;
   }
   int lo, hi, kv_lo;
   if (!split_range(ctx, p.window, p.chunk, split, lo, hi, kv_lo)) {
@@ -660,7 +662,8 @@ extern "C" int dlb_paged_decode_rows(const void* q, const void* k_cache, const v
   p.bt_stride = bt_stride;
   p.table_rows = table_rows;
   p.num_table_rows = (int)num_table_rows;
-  p.rows_is_int64 = rows_is_int64;
+  p.rows_is_int64 = rows_is_int64 & 1;
+  p.rows_gathered = rows_is_int64 & 2;
   p.batch = (int)batch;
   p.hq = (int)hq;
   p.hkv = (int)hkv;

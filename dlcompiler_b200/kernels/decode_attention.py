@@ -39,14 +39,20 @@ def decode_attention_fwd(
     assert D % 8 == 0 and Dv % 8 == 0 and D <= 128 and Dv <= 128, "head sizes: multiples of 8 up to 128"
     assert q.stride(-1) == 1 and o.stride(-1) == 1 and k_buffer.stride(-1) == 1 and v_buffer.stride(-1) == 1
     hkv = k_buffer.shape[1]
-    # the kernel looks its row up itself: gathering the rows of 16 requests of up to 32768 tokens first took 17 us of 234
-    table = req_to_token if req_to_token.dtype in (torch.int32, torch.int64) else req_to_token.to(torch.int64)
-    if table.stride(1) != 1:
-        table = table.contiguous()
     rows = b_req_idx if b_req_idx.dtype in (torch.int32, torch.int64) else b_req_idx.to(torch.int64)
     rows = rows.reshape(-1).contiguous()
     assert rows.size(0) >= batch, "b_req_idx: one table row per request"
-    max_ctx = max(min(int(max_len_in_batch), table.size(1)) if max_len_in_batch else table.size(1), 1)
+    max_ctx = max(min(int(max_len_in_batch), req_to_token.size(1)) if max_len_in_batch else req_to_token.size(1), 1)
+    if req_to_token.dtype in (torch.int32, torch.int64) and req_to_token.stride(1) == 1:
+        # the kernel looks its row up itself: gathering the rows of 16 requests of up to 32768 tokens first took 17 us of 234
+        table, gathered = req_to_token, 0
+    else:
+        # a table that it cannot read in place: only the rows and columns in use are copied, not the whole pool (int16,
+        # 4096 x 32768, 16 requests of 2048 tokens: 423 us for the pool, 74 so); the kernel still says which rows exist
+        table = req_to_token[:, :max_ctx].index_select(0, rows.clamp(0, req_to_token.size(0) - 1))
+        if table.dtype not in (torch.int32, torch.int64):
+            table = table.to(torch.int32 if table.element_size() < 4 and not table.is_floating_point() else torch.int64)
+        gathered = 2
     lens = b_seq_len if b_seq_len.dtype in (torch.int32, torch.int64) else b_seq_len.to(torch.int64)
     lens = lens.contiguous()
     chunk = _pick_chunk(batch, hkv, max_ctx, 1)
@@ -58,7 +64,7 @@ def decode_attention_fwd(
     with _lib.on_device(dev):
         rc = lib.dlb_paged_decode_rows(
             q.data_ptr(), k_buffer.data_ptr(), v_buffer.data_ptr(), o.data_ptr(), table.data_ptr(), rows.data_ptr(),
-            table.size(0), int(rows.dtype == torch.int64), lens.data_ptr(),
+            req_to_token.size(0), int(rows.dtype == torch.int64) + gathered, lens.data_ptr(),
             partial.data_ptr(), batch, head, hkv, D, Dv, 1, k_buffer.size(0), max_ctx,
             q.stride(0), q.stride(1), o.stride(0), o.stride(1),
             k_buffer.stride(0), k_buffer.stride(0), k_buffer.stride(1),

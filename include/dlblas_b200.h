@@ -268,7 +268,8 @@ int dlb_paged_decode(const void* q, const void* k_cache, const void* v_cache, vo
                      float softcap, int dtype, int32_t* status, void* stream);
 
 /* The same with one more indirection: sequence b reads row table_rows[b] (int32 or int64) of block_table instead of
- * row b; table_rows == NULL is dlb_paged_decode.  A row outside [0, num_table_rows) reads nothing: its sequence gets
+ * row b; table_rows == NULL is dlb_paged_decode.  With 2 added to rows_is_int64 the named rows have been gathered in the
+ * order of the batch: sequence b reads row b, and table_rows only says which rows exist.  A row outside [0, num_table_rows) reads nothing: its sequence gets
  * zeros and `status` the code 2 with {sequence, num_table_rows, the row}. */
 int dlb_paged_decode_rows(const void* q, const void* k_cache, const void* v_cache, void* out,
                           const void* block_table, const void* table_rows, int64_t num_table_rows,

@@ -50,3 +50,29 @@ def test_row_outside_the_table(cuda_device, bad, idx_dtype, ctx):
         check_device_status()
     assert torch.equal(outs[1][1], torch.zeros_like(q[1]))
     assert torch.equal(outs[1][[0, 2]], outs[0][[0, 2]])
+
+
+@pytest.mark.parametrize("kind", ["int16", "transposed", "every other column"])
+def test_table_that_needs_a_copy(cuda_device, kind):
+    """Bit for bit the table in its plain form, only the rows and columns in use copied: less new memory than the pool."""
+    g = torch.Generator().manual_seed(9)
+    rows, ctx, cols = 512, 300, 4096
+    pool = torch.randint(0, 5000, (rows, cols), generator=g, dtype=torch.int32).to(cuda_device)
+    table = {"int16": pool.to(torch.int16), "transposed": pool.t().contiguous().t(),
+             "every other column": pool.repeat_interleave(2, 1)[:, ::2]}[kind]
+    k, v = (torch.randn(5000, 2, 64, generator=g).to(torch.bfloat16).to(cuda_device) for _ in range(2))
+    q = torch.randn(4, 8, 64, generator=g).to(torch.bfloat16).to(cuda_device)
+    lens = torch.tensor([ctx, 1, 65, 257], dtype=torch.int32, device=cuda_device)
+    idx = torch.tensor([511, 0, -1, 511], device=cuda_device)
+    outs = []
+    for t in (pool, table):
+        o = torch.empty_like(q)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        held = torch.cuda.memory_allocated()
+        decode_attention_fwd(q, k, v, o, t, idx, None, lens, None, ctx, 0.125)
+        assert torch.cuda.max_memory_allocated() - held < rows * cols
+        with pytest.raises(DlblasError, match="request 2 "):
+            check_device_status()
+        outs.append(o)
+    assert torch.equal(outs[0], outs[1]) and not outs[0][2].any()
