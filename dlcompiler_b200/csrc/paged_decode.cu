@@ -616,8 +616,6 @@ extern "C" int dlb_paged_decode_rows(const void* q, const void* k_cache, const v
                                      void* stream) {
   DLB_NVTX("dlb_paged_decode");
   using namespace dlb;
-  DLB_CHECK_ARG(table_rows == nullptr || (num_table_rows >= 1 && num_table_rows < (1LL << 31)), DLB_ERR_BAD_ARG,
-                "paged_decode: table of %lld rows", (long long)num_table_rows);
   DLB_CHECK_ARG(dtype == DLB_DTYPE_BF16 || dtype == DLB_DTYPE_F16, DLB_ERR_UNSUPPORTED,
                 "paged_decode: dtype %d (need fp16 or bf16)", dtype);
   DLB_CHECK_ARG(head_dim >= 8 && head_dim <= 128 && head_dim % 8 == 0 && head_dim_v >= 8 && head_dim_v <= 128 &&
@@ -636,6 +634,8 @@ extern "C" int dlb_paged_decode_rows(const void* q, const void* k_cache, const v
   DLB_CHECK_ARG(batch <= 65535 && hkv * ((hq / hkv + 15) / 16) <= 65535, DLB_ERR_TOO_LARGE,
                 "paged_decode: grid too large");
   if (batch == 0) return DLB_OK;
+  DLB_CHECK_ARG(table_rows == nullptr || (num_table_rows >= 1 && num_table_rows < (1LL << 31)), DLB_ERR_BAD_ARG,
+                "paged_decode: table of %lld rows", (long long)num_table_rows);
   DLB_CHECK_ARG(q && k_cache && v_cache && out && block_table && kv_seqlens, DLB_ERR_BAD_ARG,
                 "paged_decode: null pointer");
   DLB_CHECK_ARG(q_stride_h % 2 == 0 && q_stride_b % 2 == 0 && ((uintptr_t)q & 3) == 0, DLB_ERR_ALIGNMENT,

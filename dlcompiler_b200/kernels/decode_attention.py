@@ -40,8 +40,10 @@ def decode_attention_fwd(
     assert q.stride(-1) == 1 and o.stride(-1) == 1 and k_buffer.stride(-1) == 1 and v_buffer.stride(-1) == 1
     hkv = k_buffer.shape[1]
     rows = b_req_idx if b_req_idx.dtype in (torch.int32, torch.int64) else b_req_idx.to(torch.int64)
+    assert rows.dim() <= 1, "b_req_idx is one-dimensional"
     rows = rows.reshape(-1).contiguous()
     assert rows.size(0) >= batch, "b_req_idx: one table row per request"
+    assert req_to_token.size(1) >= 1, "req_to_token has no columns"
     max_ctx = max(min(int(max_len_in_batch), req_to_token.size(1)) if max_len_in_batch else req_to_token.size(1), 1)
     if req_to_token.dtype in (torch.int32, torch.int64) and req_to_token.stride(1) == 1:
         # the kernel looks its row up itself: gathering the rows of 16 requests of up to 32768 tokens first took 17 us of 234

@@ -74,6 +74,16 @@ def test_argument_errors_are_reported_without_a_device():
     assert rc < 0 and b"experts" in lib.dlb_last_error()
 
 
+def test_decode_over_an_empty_request_table():
+    """No request asks nothing of the table; one that does is refused before any launch."""
+    lib = _lib.load()
+    for batch, want in ((0, 0), (1, -1)):
+        rc = lib.dlb_paged_decode_rows(16, 16, 16, 16, 16, 16, 0, 0, 16, None, batch, 8, 2, 64, 64, 1, 64, 1, 512, 64, 512, 64,
+                                       128, 128, 64, 128, 128, 64, 1, 0, 0, 256, 1, -1, 1.0, -1.0, _lib.DTYPE_BF16, None, None)
+        assert rc == want, lib.dlb_last_error()
+    assert b"table of 0 rows" in lib.dlb_last_error()
+
+
 def test_wrappers_refuse_cpu_tensors():
     import torch
 

@@ -31,3 +31,21 @@ def test_align_capacity_covers_the_worst_case():
         assert cap >= numel + experts * (block - 1)          # every expert may waste block - 1 entries
         assert cap - (numel + experts * (block - 1)) < block
 
+
+
+def test_decode_attention_refuses_what_names_no_row(monkeypatch):
+    """Before any launch: a two-dimensional b_req_idx, too few of them, a table without columns."""
+    import pytest
+    import torch
+
+    from dlcompiler_b200 import _lib
+    from dlcompiler_b200.kernels.decode_attention import decode_attention_fwd
+
+    monkeypatch.setattr(_lib, "require_cuda", lambda *t: torch.device("cpu"))
+    monkeypatch.setattr(_lib, "load", lambda: pytest.fail("not refused"))
+    q, kv, table = torch.zeros(4, 8, 64), torch.zeros(16, 2, 64), torch.zeros(3, 16, dtype=torch.int32)
+    lens = torch.ones(4, dtype=torch.int32)
+    for t, idx in ((table, torch.zeros(2, 2, dtype=torch.int32)), (table, torch.zeros(3, dtype=torch.int32)),
+                   (table[:, :0], torch.zeros(4, dtype=torch.int32))):
+        with pytest.raises(AssertionError, match="b_req_idx|columns"):
+            decode_attention_fwd(q, kv, kv, q, t, idx, None, lens, None, 16, 0.125)
