@@ -458,7 +458,9 @@ extern "C" int dlb_ep_route(const void* topk_ids, int ids_are_int64, int64_t num
   p.status = status;
   p.budget_ns = wait_budget_ns();
   const size_t smem = sizeof(int32_t) * (size_t)experts * (6 + ep::PLAN_THREADS / 32);
-  cudaError_t e = cudaFuncSetAttribute(ep_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  // the limit belongs to the process: always the most any call takes, so that threads do not lower it for one another
+  constexpr size_t max_smem = sizeof(int32_t) * (size_t)ep::MAX_EXPERTS * (6 + ep::PLAN_THREADS / 32);
+  cudaError_t e = cudaFuncSetAttribute(ep_route_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e != cudaSuccess) {
     set_last_error("ep_route: smem attribute: %s", cudaGetErrorString(e));
     return (int)e;

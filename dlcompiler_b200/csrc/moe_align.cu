@@ -203,7 +203,7 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   using namespace dlb;
   DLB_CHECK_ARG(numel >= 0 && numel < (1LL << 30), DLB_ERR_TOO_LARGE, "moe_align: numel=%lld out of range",
                 (long long)numel);
-  DLB_CHECK_ARG(num_experts >= 1 && num_experts <= 1024, DLB_ERR_UNSUPPORTED, "moe_align: experts=%d not in [1,1024]",
+  DLB_CHECK_ARG(num_experts >= 1 && num_experts <= SORT_MAX_EXPERTS, DLB_ERR_UNSUPPORTED, "moe_align: experts=%d not in [1,1024]",
                 num_experts);
   DLB_CHECK_ARG(block >= 1, DLB_ERR_BAD_ARG, "moe_align: block=%d", block);
   DLB_CHECK_ARG(sorted_token_ids && num_tokens_post_padded && block_start, DLB_ERR_BAD_ARG,
@@ -217,15 +217,16 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   DLB_CHECK_ARG(expert_ids == nullptr || expert_ids_capacity >= (need + block - 1) / block, DLB_ERR_BAD_ARG,
                 "moe_align: expert_ids capacity %lld too small", (long long)expert_ids_capacity);
   const size_t smem = sizeof(int32_t) * sort_smem_ints(num_experts);
+  constexpr size_t max_smem = sizeof(int32_t) * sort_smem_ints(SORT_MAX_EXPERTS);
   const int ctas = sort_cluster_size(numel);
   cudaStream_t s = (cudaStream_t)stream;
   cudaError_t e;
   if (ids_are_int64)
-    e = launch_one_cluster(moe_align_kernel<int64_t>, ctas, smem, s, (const int64_t*)topk_ids, sorted_token_ids,
+    e = launch_one_cluster(moe_align_kernel<int64_t>, ctas, smem, max_smem, s, (const int64_t*)topk_ids, sorted_token_ids,
                            expert_ids, num_tokens_post_padded, block_start, (int)numel, num_experts, block,
                            (int)sorted_capacity, (int)expert_ids_capacity);
   else
-    e = launch_one_cluster(moe_align_kernel<int32_t>, ctas, smem, s, (const int32_t*)topk_ids, sorted_token_ids,
+    e = launch_one_cluster(moe_align_kernel<int32_t>, ctas, smem, max_smem, s, (const int32_t*)topk_ids, sorted_token_ids,
                            expert_ids, num_tokens_post_padded, block_start, (int)numel, num_experts, block,
                            (int)sorted_capacity, (int)expert_ids_capacity);
   if (e != cudaSuccess) {

@@ -662,9 +662,10 @@ static int launch_gshard_assign(const float* gates, const int32_t* ids_km, const
                                 int32_t* loc, float* me, float* ce, float* l_aux, int32_t* ec_idx, float* weights,
                                 int64_t* select, int64_t tokens, int experts, int top_k, int64_t capacity,
                                 cudaStream_t stream) {
+  constexpr size_t max_smem = sizeof(int32_t) * (sort_smem_ints(SORT_MAX_EXPERTS) + 2 * (size_t)SORT_MAX_EXPERTS);
   const size_t smem = sizeof(int32_t) * (sort_smem_ints(experts) + 2 * (size_t)experts);
-  const cudaError_t e = launch_one_cluster(gshard_assign_kernel, sort_cluster_size(tokens * top_k), smem, stream, gates,
-                                           ids_km, part, (int)rows, loc, me, ce, l_aux, ec_idx, weights, select,
+  const cudaError_t e = launch_one_cluster(gshard_assign_kernel, sort_cluster_size(tokens * top_k), smem, max_smem,
+                                           stream, gates, ids_km, part, (int)rows, loc, me, ce, l_aux, ec_idx, weights, select,
                                            (int)tokens, experts, top_k, (int)capacity, 1.1920928955078125e-07f);
   if (e != cudaSuccess) {
     set_last_error("gshard_assign: launch: %s", cudaGetErrorString(e));
@@ -821,7 +822,7 @@ extern "C" int dlb_gshard_assign(const float* gates, const int32_t* ids_choice_m
   using namespace dlb;
   (void)sorted_slots;       // the launch sorts the slots itself
   (void)expert_prefix;
-  DLB_CHECK_ARG(tokens >= 1 && experts >= 1 && experts <= 1024 && top_k >= 1 && capacity >= 1 && colsum_blocks >= 1,
+  DLB_CHECK_ARG(tokens >= 1 && experts >= 1 && experts <= SORT_MAX_EXPERTS && top_k >= 1 && capacity >= 1 && colsum_blocks >= 1,
                 DLB_ERR_BAD_ARG, "gshard_assign: bad sizes");
   DLB_CHECK_ARG(tokens * top_k < (1LL << 30) && (int64_t)experts * capacity < (1LL << 31), DLB_ERR_TOO_LARGE,
                 "gshard_assign: problem too large");

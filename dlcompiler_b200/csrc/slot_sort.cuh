@@ -29,7 +29,8 @@ inline int sort_cluster_size(int64_t numel) {
 }
 // Row pitch of the table: odd, so that a column walk touches 32 different banks.
 __host__ __device__ constexpr int sort_pitch(int experts) { return experts | 1; }
-inline size_t sort_smem_ints(int experts) {
+constexpr int SORT_MAX_EXPERTS = 1024;
+constexpr size_t sort_smem_ints(int experts) {
   return (size_t)SORT_WARPS * sort_pitch(experts) + 4 * (size_t)experts + 1 + 2 * SORT_WARPS;
 }
 
@@ -170,11 +171,13 @@ struct SlotSort {
   }
 };
 
-// Launches `kern` as one cluster of `ctas` CTAs with `smem` bytes of dynamic shared memory.
+// Launches `kern` as one cluster of `ctas` CTAs with `smem` bytes of dynamic shared memory.  The kernel's limit is set to
+// `max_smem`, the most that any call of it takes: the limit belongs to the process, and a call that set it to its own
+// need could lower it between another thread's setting and launch.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_one_cluster(void (*kern)(KArgs...), int ctas, size_t smem, cudaStream_t stream,
-                                      Args... args) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+inline cudaError_t launch_one_cluster(void (*kern)(KArgs...), int ctas, size_t smem, size_t max_smem,
+                                      cudaStream_t stream, Args... args) {
+  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)max_smem);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);

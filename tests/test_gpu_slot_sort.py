@@ -1,9 +1,12 @@
 """GPU: the cluster-wide slot sort at the edges of its cluster sizes, segments and expert counts (integers: exact)."""
+import threading
+from ctypes import c_int, c_int64, c_void_p
+
 import pytest
 import torch
 
-from dlcompiler_b200 import topk_gating
-from dlcompiler_b200.kernels.fused_moe import _moe_align
+from dlcompiler_b200 import _lib, topk_gating
+from dlcompiler_b200.kernels.fused_moe import _align_capacity, _moe_align
 from oracle import dlblas_oracle as oracle
 
 pytestmark = pytest.mark.gpu
@@ -31,3 +34,30 @@ def test_gate_at_cluster_edges(cuda_device, S, E, k, cf):
     assert torch.equal(ec.cpu(), rec) and torch.equal(sel.cpu(), rsel)
     torch.testing.assert_close(l_aux.cpu(), rl, rtol=1e-5, atol=1e-6)
     torch.testing.assert_close(w.cpu(), rw, rtol=1e-5, atol=1e-7)
+
+
+def test_threads_with_different_expert_counts(cuda_device):
+    """The kernel's shared-memory limit is one for the process: a thread with few experts must not lower it for a launch
+    with many (1024 experts take 148 KB, 8 take 1.4).  The entry point itself in a tight loop, which holds no lock."""
+    lib = _lib.load()
+    codes = []
+
+    def work(E):
+        cap = _align_capacity(64, E, 8)
+        buf = torch.zeros(2 * cap + E + 2 + 64, dtype=torch.int32, device=cuda_device)
+        at = [buf.data_ptr() + 4 * o for o in (0, 64, 64 + cap, 64 + 2 * cap, 65 + 2 * cap)]
+        call = [c_void_p(at[0]), c_int(0), c_int64(64), c_int(E), c_int(8), c_void_p(at[1]), c_int64(cap), c_void_p(at[2]),
+                c_int64(cap), c_void_p(at[3]), c_void_p(at[4]), c_void_p(stream.cuda_stream)]
+        start.wait()
+        codes.extend({fn(*call) for _ in range(20000)})
+        stream.synchronize()
+
+    stream, start = torch.cuda.Stream(), threading.Barrier(4)
+    fn = lib.dlb_moe_align_block_size
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(E,)) for E in (8, 1024, 16, 1000)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert set(codes) == {0}
