@@ -40,17 +40,21 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_align_kernel(
     const int pos = first[e] * block + at;
     if (pos < sorted_capacity) sorted_token_ids[pos] = slot;
   });
-  // what no slot fills: each expert's padding, the list behind the last block, and the block owners
+  // what no slot fills: each expert's padding, the list behind the last block, and the block owners.  The capacity may
+  // come up to 2^31 - 1: unsigned, so that the step past it does not turn negative and write on.
+  static_assert(0x7fffffffu + SORT_MAX_CLUSTER * SORT_THREADS > 0x7fffffffu);
   const int tid = sort.rank * SORT_THREADS + threadIdx.x, threads = sort.ctas * SORT_THREADS;
   if (block > 1) {
     const int lane = threadIdx.x & 31;
     for (int e = tid >> 5; e < num_experts; e += threads >> 5)
-      for (int i = first[e] * block + sort.count[e] + lane; i < min(first[e + 1] * block, sorted_capacity); i += 32)
+      for (unsigned i = first[e] * block + sort.count[e] + lane; i < (unsigned)min(first[e + 1] * block, sorted_capacity);
+           i += 32)
         sorted_token_ids[i] = numel;
   }
-  for (int i = blocks * block + tid; i < sorted_capacity; i += threads) sorted_token_ids[i] = numel;
+  for (unsigned i = blocks * block + tid; i < (unsigned)sorted_capacity; i += threads) sorted_token_ids[i] = numel;
   if (expert_ids != nullptr) {
-    for (int b = tid; b < expert_ids_capacity; b += threads) {
+    for (int64_t i = tid; i < expert_ids_capacity; i += threads) {
+      const int b = (int)i;
       int lo = 0, hi = num_experts;      // last expert whose first block is <= b (empty ones share it with the next)
       while (hi - lo > 1) {
         const int mid = (lo + hi) >> 1;
