@@ -461,7 +461,10 @@ grouped_topk_kernel(GatingParams p) {
       my_v = pick;
     }
   }
-  const int my_id = my_owner * VPL + my_v;
+  int my_id = my_owner * VPL + my_v;
+  // the -inf fillers of a ragged last lane rank above a negative NaN: where the id indexes the probabilities afterwards
+  // (the capacity-limited gate) it has to be one of the experts
+  if (!FULL && p.probs != nullptr) my_id = min(my_id, E - 1);
   if constexpr (GATE) {
     if (live && lane < top_k) p.ids[(int64_t)lane * p.tokens + token] = my_id;
     return;

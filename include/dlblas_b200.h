@@ -67,7 +67,7 @@ int dlb_grouped_topk_gating(const float* logits, const float* bias, int32_t* ids
  * topk_gating_bwd.py:20-85; torch statement python/dlBLAS/benchmarks/topk_gating.py:132-206.
  *   dlb_gshard_gate     gates = softmax(logits) [tokens, experts] fp32 and the k largest experts per token
  *                       (ids [tokens, top_k], descending, ties to the lower index).
- *   dlb_gshard_assign   from the choice-major id list [top_k * tokens]: queue position of every choice (loc),
+ *   dlb_gshard_assign   from the choice-major id list [top_k * tokens] (ids in [0, experts)): queue position of every choice (loc),
  *                       me / ce / l_aux = mean(me * ce) * E^2, kept choices (position < capacity),
  *                       weights = kept gate / max(sum of the token's kept gates, fp32 eps),
  *                       ec_idx = expert * capacity + position (0 when dropped),

@@ -36,6 +36,22 @@ def test_gate_at_cluster_edges(cuda_device, S, E, k, cf):
     torch.testing.assert_close(w.cpu(), rw, rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("E,k", [(8, 8), (5, 3), (40, 20)])
+def test_gate_of_a_negative_nan(cuda_device, E, k):
+    """The fillers of a ragged gate rank above it: no id outside the experts, forward and backward (nothing reads or
+    writes outside the gates), and the other tokens' gradients stay finite."""
+    logits = torch.randn(37, E, generator=torch.Generator().manual_seed(E))
+    logits[3] = torch.tensor(-1, dtype=torch.int32).view(torch.float32)
+    logits[36, ::2] = torch.tensor(-4194304, dtype=torch.int32).view(torch.float32)
+    x = logits.to(cuda_device).requires_grad_()
+    _, ec, w, sel = topk_gating(x, k, 1.0, 2, True)
+    ids = w.grad_fn.saved_tensors[2]
+    assert ((ids >= 0) & (ids < E)).all()
+    w.nan_to_num().sum().backward()
+    assert ((ec >= 0) & (ec < sel.numel())).all() and ((sel >= 0) & (sel < 37)).all()
+    assert torch.isfinite(x.grad[[i for i in range(36) if i != 3]]).all()
+
+
 def test_threads_with_different_expert_counts(cuda_device):
     """The kernel's shared-memory limit is one for the process: a thread with few experts must not lower it for a launch
     with many (1024 experts take 148 KB, 8 take 1.4).  The entry point itself in a tight loop, which holds no lock."""
