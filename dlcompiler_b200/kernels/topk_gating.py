@@ -17,7 +17,11 @@ def _f32(x: float) -> float:
 def _capacity(num_tokens: int, num_experts: int, capacity_factor: float, min_capacity: int) -> int:
     """ceil(tokens / experts * capacity_factor), at least min_capacity (topk_gating.py:13-22; the product is
     formed with an fp32 tensor there, reproduced here so the integer agrees)."""
-    cap = math.ceil(_f32(_f32(num_tokens / num_experts) * _f32(capacity_factor)))
+    cap = _f32(_f32(num_tokens / num_experts) * _f32(capacity_factor))
+    if abs(cap) < 2.0**31:
+        return max(math.ceil(cap), int(min_capacity))
+    # NaN, infinite or past any capacity: whatever the tensor's own conversion to int64 makes of it
+    cap = torch.ceil((num_tokens / num_experts) * torch.tensor(capacity_factor)).to(torch.int64)
     return max(int(cap), int(min_capacity))
 
 

@@ -49,3 +49,27 @@ def test_decode_attention_refuses_what_names_no_row(monkeypatch):
                    (table[:, :0], torch.zeros(4, dtype=torch.int32))):
         with pytest.raises(AssertionError, match="b_req_idx|columns"):
             decode_attention_fwd(q, kv, kv, q, t, idx, None, lens, None, 16, 0.125)
+
+
+def test_gate_capacity_is_the_tensor_arithmetic():
+    """The fp32 product of the tensor form, rounding, infinities, NaN and refusals included."""
+    import math
+    import random
+
+    import pytest
+    import torch
+
+    from dlcompiler_b200.kernels.topk_gating import _capacity
+
+    def tensor_form(tokens, experts, factor, least):
+        return max(int(torch.ceil((tokens / experts) * torch.tensor(factor)).to(torch.int64)), int(least))
+
+    r = random.Random(0)
+    cases = [(64, 8, f, 4) for f in (math.inf, -math.inf, math.nan, 1e30, -1e30, 1e300, 2.0**31, 9.3e18, -3.0, 0.0, 2, True)]
+    cases += [(r.randint(1, 1 << r.randint(1, 21)), r.randint(1, 512), r.choice([r.random() * 8, r.randint(1, 32) * 1.1,
+                                                                                r.randint(1, 32) / 3, 1.25]), 2)
+              for _ in range(3000)]
+    for case in cases:
+        assert _capacity(*case) == tensor_form(*case), case
+    with pytest.raises(ValueError):
+        _capacity(64, 8, 2**70, 4)
