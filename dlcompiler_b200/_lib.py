@@ -17,7 +17,7 @@ LIB_PATH = os.path.join(_PKG_DIR, "libdlblas_b200.so")
 DTYPE_F16, DTYPE_BF16, DTYPE_F32 = 0, 1, 2
 SCORE_SIGMOID, SCORE_SOFTMAX = 0, 1
 DEV_BAD_ROW = 2  # code in a device status word
-GEMM_FUSE_SILU, GEMM_WEIGHT, GEMM_SCATTER, GEMM_PEER = 1, 2, 4, 8
+GEMM_FUSE_SILU, GEMM_WEIGHT, GEMM_SCATTER, GEMM_PEER, GEMM_SLOTS_ONLY = 1, 2, 4, 8, 16
 
 _DTYPES = {torch.float16: DTYPE_F16, torch.bfloat16: DTYPE_BF16, torch.float32: DTYPE_F32}
 
@@ -42,6 +42,8 @@ SIGNATURES = {
                                          c_int64, c_void_p, c_void_p, c_void_p]),
     "dlb_moe_permute_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int64, c_int64,
                                      c_int64, c_int, c_void_p]),
+    "dlb_moe_permute_slots": (c_int, [c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int, c_int64, c_int64,
+                                      c_int64, c_int, c_void_p]),
     "dlb_moe_grouped_gemm": (c_int, [c_void_p, c_int64, c_int64, c_void_p, c_int, c_int64, c_int64, c_int64,
                                      c_void_p, c_int64, c_int64, c_void_p, c_void_p, c_void_p, c_int64, c_int,
                                      c_int, c_void_p, c_void_p]),

@@ -57,6 +57,7 @@ constexpr int FLAG_FUSE_SILU = 1;
 constexpr int FLAG_WEIGHT = 2;
 constexpr int FLAG_SCATTER = 4;
 constexpr int FLAG_PEER = 8;       // scatter to (rank, slot) taken from row_meta: plain stores into peer memory
+constexpr int FLAG_SLOTS_ONLY = 16; // rows of no slot may be left unstored; read by the host only
 constexpr int MAX_PEERS = 16;
 }  // namespace gg
 
@@ -506,6 +507,10 @@ static int grouped_gemm_impl(const void* a, int64_t a_rows, int64_t a_row_stride
   DLB_CHECK_ARG(k < (1LL << 31) && n_out < (1LL << 31) && a_rows < (1LL << 31) && numel < (1LL << 31) &&
                     (int64_t)num_experts * rows_per_expert < (1LL << 31),
                 DLB_ERR_TOO_LARGE, "grouped_gemm: a dimension exceeds int32");
+  // Without SCATTER every row of the blocks is a result and sorted_token_ids need not tell them apart: the form that
+  // trims A to the slots' rows is for callers that say so.
+  const bool slots_only = (flags & (FLAG_SLOTS_ONLY | FLAG_SCATTER)) != 0;
+  flags &= ~FLAG_SLOTS_ONLY;
   const bool silu = (flags & FLAG_FUSE_SILU) != 0;
   if (silu) {
     DLB_CHECK_ARG(flags == FLAG_FUSE_SILU, DLB_ERR_UNSUPPORTED, "grouped_gemm: silu fusion excludes weight/scatter");
@@ -573,10 +578,10 @@ static int grouped_gemm_impl(const void* a, int64_t a_rows, int64_t a_row_stride
   const bool bf = dtype == DLB_DTYPE_BF16;
   // Padding a third of the row list or more: few rows per block, the launch waits for the weights, and whole boxes of
   // A would add half of their bytes.  With full blocks the tensor cores' power is the limit and the few rows of padding
-  // had better be the zeros that moe_permute_rows makes them.
+  // had better be the zeros that moe_permute_slots makes them.
   // Measured, whole fused_moe, before -> after: 32 tokens over 8 experts (4096 x 14336) 503 -> 477 us, 2000 over 256
   // (2048 x 1024) 773 -> 687, 128 over 64 (2048 x 1408) 265 -> 248, 4096 over 32 (1024 x 2816) 575 -> 547.
-  if ((a_rows - numel) * 2 >= numel) {
+  if (slots_only && (a_rows - numel) * 2 >= numel) {
     if (flags == FLAG_FUSE_SILU)
       return bf ? launch_grouped<__nv_bfloat16, FLAG_FUSE_SILU, true>(ta, tb, p, grid, s)
                 : launch_grouped<__half, FLAG_FUSE_SILU, true>(ta, tb, p, grid, s);

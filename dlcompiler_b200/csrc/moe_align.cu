@@ -241,12 +241,10 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   return DLB_OK;
 }
 
-extern "C" int dlb_moe_permute_rows(const void* src, void* dst, const int32_t* sorted_token_ids,
-                                    const int32_t* num_tokens_post_padded, int64_t numel, int top_k,
-                                    int64_t hidden, int64_t src_row_stride, int64_t sorted_capacity,
-                                    int elem_size, void* stream) {
-  DLB_NVTX("dlb_moe_permute_rows");
-  using namespace dlb;
+namespace dlb {
+static int permute_rows(const void* src, void* dst, const int32_t* sorted_token_ids,
+                        const int32_t* num_tokens_post_padded, int64_t numel, int top_k, int64_t hidden,
+                        int64_t src_row_stride, int64_t sorted_capacity, int elem_size, bool zero_padding, void* stream) {
   DLB_CHECK_ARG(elem_size == 2 || elem_size == 4, DLB_ERR_UNSUPPORTED, "moe_permute: element size %d", elem_size);
   DLB_CHECK_ARG(top_k >= 1 && numel >= 0 && hidden >= 0, DLB_ERR_BAD_ARG, "moe_permute: bad sizes");
   if (sorted_capacity == 0 || hidden == 0) return DLB_OK;
@@ -261,9 +259,28 @@ extern "C" int dlb_moe_permute_rows(const void* src, void* dst, const int32_t* s
   moe_permute_rows_kernel<<<(unsigned)blocks, 256, 0, (cudaStream_t)stream>>>(
       (const uint4*)src, (uint4*)dst, sorted_token_ids, num_tokens_post_padded, (int)numel, top_k,
       (int)(row_bytes / 16), src_row_stride * elem_size / 16, (int)sorted_capacity,
-      (sorted_capacity - numel) * 2 < numel ? 1 : 0);      // the grouped GEMM's rule for whole boxes of A
+      zero_padding ? 1 : 0);
   DLB_CUDA_LAUNCH_CHECK();
   return DLB_OK;
+}
+}  // namespace dlb
+
+extern "C" int dlb_moe_permute_rows(const void* src, void* dst, const int32_t* sorted_token_ids,
+                                    const int32_t* num_tokens_post_padded, int64_t numel, int top_k,
+                                    int64_t hidden, int64_t src_row_stride, int64_t sorted_capacity,
+                                    int elem_size, void* stream) {
+  DLB_NVTX("dlb_moe_permute_rows");
+  return dlb::permute_rows(src, dst, sorted_token_ids, num_tokens_post_padded, numel, top_k, hidden, src_row_stride,
+                           sorted_capacity, elem_size, true, stream);
+}
+
+extern "C" int dlb_moe_permute_slots(const void* src, void* dst, const int32_t* sorted_token_ids,
+                                     const int32_t* num_tokens_post_padded, int64_t numel, int top_k,
+                                     int64_t hidden, int64_t src_row_stride, int64_t sorted_capacity,
+                                     int elem_size, void* stream) {
+  DLB_NVTX("dlb_moe_permute_slots");
+  return dlb::permute_rows(src, dst, sorted_token_ids, num_tokens_post_padded, numel, top_k, hidden, src_row_stride,
+                           sorted_capacity, elem_size, (sorted_capacity - numel) * 2 < numel, stream);   // the GEMM's rule
 }
 
 extern "C" int dlb_moe_combine(const void* partial, void* out, int64_t tokens, int top_k, int64_t hidden,

@@ -61,7 +61,8 @@ class CudaOps:
         cap = sorted_ids.numel()
         a_sorted = _permute_rows(rows, sorted_ids, num_post, R, 1, cap)
         act = torch.empty((cap, N // 2), dtype=rows.dtype, device=rows.device)
-        fm._grouped_gemm(a_sorted, w1, act, N // 2, sorted_ids, block_start, None, R, _lib.GEMM_FUSE_SILU)
+        fm._grouped_gemm(a_sorted, w1, act, N // 2, sorted_ids, block_start, None, R,
+                         _lib.GEMM_FUSE_SILU | _lib.GEMM_SLOTS_ONLY)
         out = torch.empty((R, w2.size(1)), dtype=rows.dtype, device=rows.device)
         fm._grouped_gemm(act, w2, out, w2.size(1), sorted_ids, block_start, weights, R,
                          _lib.GEMM_WEIGHT | _lib.GEMM_SCATTER)

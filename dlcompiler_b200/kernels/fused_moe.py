@@ -56,14 +56,15 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: i
 
 
 def _permute_rows(src, row_map, num_post, numel, div, cap):
+    """Rows of `src` in the order of `row_map`; rows of no slot may be left as they are."""
     hidden = src.size(-1)
     dst = torch.empty((cap, hidden), dtype=src.dtype, device=src.device)
     lib = _lib.load()
     with _lib.on_device(src.device):
-        rc = lib.dlb_moe_permute_rows(src.data_ptr(), dst.data_ptr(), row_map.data_ptr(), num_post.data_ptr(), numel,
-                                      div, hidden, src.stride(0), cap, src.element_size(),
-                                      _lib.stream_ptr(src.device))
-    _lib.check(rc, "moe_permute_rows")
+        rc = lib.dlb_moe_permute_slots(src.data_ptr(), dst.data_ptr(), row_map.data_ptr(), num_post.data_ptr(), numel,
+                                       div, hidden, src.stride(0), cap, src.element_size(),
+                                       _lib.stream_ptr(src.device))
+    _lib.check(rc, "moe_permute_slots")
     return dst
 
 
@@ -134,7 +135,8 @@ def fused_moe(hidden_states: torch.Tensor,
 
     a_sorted = _permute_rows(hidden_states, sorted_ids, num_post, numel, topk, cap)
     act = torch.empty((cap, inter), dtype=hidden_states.dtype, device=dev)
-    _grouped_gemm(a_sorted, w1, act, inter, sorted_ids, block_start, None, numel, _lib.GEMM_FUSE_SILU)
+    _grouped_gemm(a_sorted, w1, act, inter, sorted_ids, block_start, None, numel,
+                  _lib.GEMM_FUSE_SILU | _lib.GEMM_SLOTS_ONLY)
     partial = torch.empty((numel, H_out), dtype=hidden_states.dtype, device=dev)
     _grouped_gemm(act, w2, partial, H_out, sorted_ids, block_start, topk_weights, numel,
                   _lib.GEMM_WEIGHT | _lib.GEMM_SCATTER)

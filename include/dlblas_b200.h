@@ -34,6 +34,7 @@ extern "C" {
 #define DLB_GEMM_FUSE_SILU 1 /* B = [gate; up] halves, store silu(gate) * up */
 #define DLB_GEMM_WEIGHT 2    /* scale each row by its routing weight (fp32) before the cast */
 #define DLB_GEMM_SCATTER 4   /* write row p to row sorted_token_ids[p] of the output */
+#define DLB_GEMM_SLOTS_ONLY 16 /* rows of no slot need not be stored (faster where there are many) */
 
 /* Library version (major * 100 + minor). */
 int dlb_version(void);
@@ -120,18 +121,24 @@ int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64, int64_t nu
 int dlb_moe_start_end(const void* topk_ids, int ids_are_int64, int64_t numel, int num_experts, void* exp_start,
                       void* exp_end, int out_is_int64, void* stream);
 
-/* dst[p, :] = src[sorted_token_ids[p] / top_k, :] for p < num_tokens_post_padded (rows of sentinel
- * entries: zeros, or left alone when the padding is a third of the capacity or more).  The gather the reference does inside its GEMM by pointer arithmetic (reindex_a,
+/* dst[p, :] = src[sorted_token_ids[p] / top_k, :] for p < num_tokens_post_padded (zeros for sentinel
+ * rows).  The gather the reference does inside its GEMM by pointer arithmetic (reindex_a,
  * python/dlBLAS/dlblas/kernels/fused_moe.py:136-140), as a separate pass so the GEMM can use TMA. */
 int dlb_moe_permute_rows(const void* src, void* dst, const int32_t* sorted_token_ids,
                          const int32_t* num_tokens_post_padded, int64_t numel, int top_k, int64_t hidden,
                          int64_t src_row_stride, int64_t sorted_capacity, int elem_size, void* stream);
 
+/* The same for a list whose sentinel rows nobody looks at: they are left alone where they are a third of
+ * sorted_capacity or more. */
+int dlb_moe_permute_slots(const void* src, void* dst, const int32_t* sorted_token_ids,
+                          const int32_t* num_tokens_post_padded, int64_t numel, int top_k, int64_t hidden,
+                          int64_t src_row_stride, int64_t sorted_capacity, int elem_size, void* stream);
+
 /* Grouped GEMM over the block-padded row list: for every 128-row block b,
  * out[rows of b] = A[rows of b] @ B[expert of b]^T (fp32 accumulate), with the epilogue chosen by
  * `flags` (DLB_GEMM_*).  A is [a_rows, k] with a_rows a multiple of 128, B is
  * [num_experts * rows_per_expert, k].  Rows whose sorted_token_ids entry is not below numel belong to no
- * slot: with SCATTER, WEIGHT or many of them they are not stored.  Replaces fused_moe_kernel and its launcher,
+ * slot: with SCATTER or WEIGHT they are not stored, with SLOTS_ONLY they may be left out.  Replaces fused_moe_kernel and its launcher,
  * python/dlBLAS/dlblas/kernels/fused_moe.py:77-175 and :178-235. */
 int dlb_moe_grouped_gemm(const void* a, int64_t a_rows, int64_t a_row_stride, const void* b, int num_experts,
                          int64_t rows_per_expert, int64_t k, int64_t b_row_stride, void* out,

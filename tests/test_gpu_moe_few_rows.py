@@ -67,7 +67,8 @@ def test_silu_of_every_value(cuda_device, dtype, few):
     ids[0] = 0
     out = torch.zeros(128, n, dtype=dtype, device=cuda_device)
     _grouped_gemm(a.to(cuda_device), w1.to(cuda_device), out, n, ids.to(cuda_device),
-                  torch.tensor([0, 1], dtype=torch.int32, device=cuda_device), None, numel, _lib.GEMM_FUSE_SILU)
+                  torch.tensor([0, 1], dtype=torch.int32, device=cuda_device), None, numel,
+                  _lib.GEMM_FUSE_SILU | _lib.GEMM_SLOTS_ONLY)
     got, x = out[0].cpu().double(), gates.double()
     ref = torch.nn.functional.silu(x)
     gone = x < -88.73
@@ -78,3 +79,29 @@ def test_silu_of_every_value(cuda_device, dtype, few):
     # the smallest normal number as the floor: the tensor cores may take a subnormal operand as zero
     torch.testing.assert_close(got[rest], ref[rest], rtol=2 * torch.finfo(dtype).eps + 2.0 ** -17,
                                atol=torch.finfo(dtype).tiny)
+
+
+def test_c_entries_keep_the_rows_of_no_slot(cuda_device):
+    """Called without SLOTS_ONLY the GEMM stores every row of its blocks, whatever sorted_token_ids holds, and the permute
+    writes zeros for the sentinel rows, however many there are."""
+    g = torch.Generator().manual_seed(2)
+    lib, stream = _lib.load(), _lib.stream_ptr(cuda_device)
+    a = torch.randn(256, 64, generator=g).to(torch.bfloat16).to(cuda_device)
+    w = (torch.randn(2, 2 * 40, 64, generator=g) * 0.2).to(torch.bfloat16).to(cuda_device)
+    starts = torch.tensor([0, 1, 2], dtype=torch.int32, device=cuda_device)
+    nobody = torch.full((256,), 1 << 30, dtype=torch.int32, device=cuda_device)
+    out = torch.full((256, 40), float("nan"), dtype=torch.bfloat16, device=cuda_device)
+    _grouped_gemm(a, w, out, 40, nobody, starts, None, 1, _lib.GEMM_FUSE_SILU)
+    h = torch.einsum("erk,enk->ern", a.view(2, 128, 64).float(), w.float()).to(torch.bfloat16).float()
+    gate = torch.nn.functional.silu(h[..., :40]).to(torch.bfloat16).float()
+    ref = (gate * h[..., 40:]).view(256, 40)
+    torch.testing.assert_close(out.float(), ref, rtol=2e-2, atol=2e-2 * float(ref.std()))
+    ids = torch.full((256,), 9, dtype=torch.int32, device=cuda_device)
+    ids[3], ids[130] = 8, 0
+    post = torch.tensor([256], dtype=torch.int32, device=cuda_device)
+    for entry, untouched in ((lib.dlb_moe_permute_rows, False), (lib.dlb_moe_permute_slots, True)):
+        dst = torch.full((256, 64), 7.0, dtype=torch.bfloat16, device=cuda_device)
+        _lib.check(entry(a.data_ptr(), dst.data_ptr(), ids.data_ptr(), post.data_ptr(), 9, 1, 64, 64, 256, 2, stream), "permute")
+        assert torch.equal(dst[3], a[8]) and torch.equal(dst[130], a[0])
+        dst[3] = dst[130] = 7.0 if untouched else 0.0
+        assert (dst == (7.0 if untouched else 0.0)).all()
