@@ -529,14 +529,24 @@ static int grouped_gemm_impl(const void* a, int64_t a_rows, int64_t a_row_stride
   }
   if (a_rows == 0) return DLB_OK;
 
-  CUtensorMap ta[2];      // one map per box height
-  GroupedGemmWeightMaps tb;
+  // Padding a third of the row list or more: few rows per block, the launch waits for the weights, and whole boxes of
+  // A would add half of their bytes.  With full blocks the tensor cores' power is the limit and the few rows of padding
+  // had better be the zeros that moe_permute_slots makes them.
+  // Measured, whole fused_moe, before -> after: 32 tokens over 8 experts (4096 x 14336) 503 -> 477 us, 2000 over 256
+  // (2048 x 1024) 773 -> 687, 128 over 64 (2048 x 1408) 265 -> 248, 4096 over 32 (1024 x 2816) 575 -> 547.
+  const bool few = slots_only && (a_rows - numel) * 2 >= numel &&
+                   (flags == FLAG_FUSE_SILU || flags == (FLAG_WEIGHT | FLAG_SCATTER));
+
+  // One map per box height of A and per tile width; the form with few rows uses them all, the other the first of each
+  // (encoding all nine takes 0.4 us of the host).
+  CUtensorMap ta[2] = {};
+  GroupedGemmWeightMaps tb = {};
   const uint32_t a_rows_box[2] = {(uint32_t)BM, (uint32_t)A_BOX_ROWS};
-  for (int i = 0; i < 2; ++i) {
+  for (int i = 0; i < (few ? 2 : 1); ++i) {
     const int rc = make_tmap_2d_16b(&ta[i], a, (uint64_t)k, (uint64_t)a_rows, (uint64_t)a_row_stride * 2, BK, a_rows_box[i]);
     if (rc != DLB_OK) return rc;
   }
-  for (int i = 0; i < WIDTHS; ++i) {
+  for (int i = 0; i < (few ? WIDTHS : 1); ++i) {
     const int rc = make_tmap_2d_16b(&tb.map[i], b, (uint64_t)k, (uint64_t)num_experts * rows_per_expert,
                                     (uint64_t)b_row_stride * 2, BK, (uint32_t)((silu ? 128 : 256) / 8 * (8 - i)));
     if (rc != DLB_OK) return rc;
@@ -576,18 +586,12 @@ static int grouped_gemm_impl(const void* a, int64_t a_rows, int64_t a_row_stride
   const int grid = sm_count(current_device());
   cudaStream_t s = (cudaStream_t)stream;
   const bool bf = dtype == DLB_DTYPE_BF16;
-  // Padding a third of the row list or more: few rows per block, the launch waits for the weights, and whole boxes of
-  // A would add half of their bytes.  With full blocks the tensor cores' power is the limit and the few rows of padding
-  // had better be the zeros that moe_permute_slots makes them.
-  // Measured, whole fused_moe, before -> after: 32 tokens over 8 experts (4096 x 14336) 503 -> 477 us, 2000 over 256
-  // (2048 x 1024) 773 -> 687, 128 over 64 (2048 x 1408) 265 -> 248, 4096 over 32 (1024 x 2816) 575 -> 547.
-  if (slots_only && (a_rows - numel) * 2 >= numel) {
+  if (few) {
     if (flags == FLAG_FUSE_SILU)
       return bf ? launch_grouped<__nv_bfloat16, FLAG_FUSE_SILU, true>(ta, tb, p, grid, s)
                 : launch_grouped<__half, FLAG_FUSE_SILU, true>(ta, tb, p, grid, s);
-    if (flags == (FLAG_WEIGHT | FLAG_SCATTER))
-      return bf ? launch_grouped<__nv_bfloat16, FLAG_WEIGHT | FLAG_SCATTER, true>(ta, tb, p, grid, s)
-                : launch_grouped<__half, FLAG_WEIGHT | FLAG_SCATTER, true>(ta, tb, p, grid, s);
+    return bf ? launch_grouped<__nv_bfloat16, FLAG_WEIGHT | FLAG_SCATTER, true>(ta, tb, p, grid, s)
+              : launch_grouped<__half, FLAG_WEIGHT | FLAG_SCATTER, true>(ta, tb, p, grid, s);
   }
   switch (flags) {
     case FLAG_FUSE_SILU:
