@@ -52,17 +52,15 @@ __global__ void __launch_bounds__(SORT_THREADS) moe_align_kernel(
         sorted_token_ids[i] = numel;
   }
   for (unsigned i = blocks * block + tid; i < (unsigned)sorted_capacity; i += threads) sorted_token_ids[i] = numel;
-  if (expert_ids != nullptr) {
-    for (int64_t i = tid; i < expert_ids_capacity; i += threads) {
-      const int b = (int)i;
-      int lo = 0, hi = num_experts;      // last expert whose first block is <= b (empty ones share it with the next)
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (first[mid] <= b) lo = mid;
-        else hi = mid;
-      }
-      expert_ids[b] = b < blocks ? lo : -1;
+  for (int64_t i = tid; i < expert_ids_capacity; i += threads) {
+    const int b = (int)i;
+    int lo = 0, hi = num_experts;      // last expert whose first block is <= b (empty ones share it with the next)
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (first[mid] <= b) lo = mid;
+      else hi = mid;
     }
+    expert_ids[b] = b < blocks ? lo : -1;
   }
   if (sort.rank == 0) {
     for (int e = threadIdx.x; e <= num_experts; e += SORT_THREADS) block_start[e] = first[e];
@@ -210,7 +208,7 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   DLB_CHECK_ARG(num_experts >= 1 && num_experts <= SORT_MAX_EXPERTS, DLB_ERR_UNSUPPORTED, "moe_align: experts=%d not in [1,1024]",
                 num_experts);
   DLB_CHECK_ARG(block >= 1, DLB_ERR_BAD_ARG, "moe_align: block=%d", block);
-  DLB_CHECK_ARG(sorted_token_ids && num_tokens_post_padded && block_start, DLB_ERR_BAD_ARG,
+  DLB_CHECK_ARG(sorted_token_ids && expert_ids && num_tokens_post_padded && block_start, DLB_ERR_BAD_ARG,
                 "moe_align: null output pointer");
   DLB_CHECK_ARG(numel == 0 || topk_ids != nullptr, DLB_ERR_BAD_ARG, "moe_align: null topk_ids");
   // worst case padded length: every expert wastes block-1 entries
@@ -218,7 +216,7 @@ extern "C" int dlb_moe_align_block_size(const void* topk_ids, int ids_are_int64,
   const int64_t need = numel == 0 ? 0 : (worst < (numel + block - 1) / block * block ? worst : worst);
   DLB_CHECK_ARG(sorted_capacity >= need && sorted_capacity < (1LL << 31), DLB_ERR_BAD_ARG,
                 "moe_align: sorted_token_ids capacity %lld < %lld", (long long)sorted_capacity, (long long)need);
-  DLB_CHECK_ARG(expert_ids == nullptr || expert_ids_capacity >= (need + block - 1) / block, DLB_ERR_BAD_ARG,
+  DLB_CHECK_ARG(expert_ids_capacity >= (need + block - 1) / block, DLB_ERR_BAD_ARG,
                 "moe_align: expert_ids capacity %lld too small", (long long)expert_ids_capacity);
   const size_t smem = sizeof(int32_t) * sort_smem_ints(num_experts);
   constexpr size_t max_smem = sizeof(int32_t) * sort_smem_ints(SORT_MAX_EXPERTS);

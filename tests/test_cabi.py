@@ -74,6 +74,14 @@ def test_argument_errors_are_reported_without_a_device():
     assert rc < 0 and b"experts" in lib.dlb_last_error()
 
 
+def test_align_needs_all_of_its_outputs():
+    lib = _lib.load()
+    for missing in range(4):
+        out = [None if i == missing else 16 for i in range(4)]
+        rc = lib.dlb_moe_align_block_size(16, 0, 8, 4, 16, out[0], 128, out[1], 8, out[2], out[3], None)
+        assert rc < 0 and b"null output" in lib.dlb_last_error()
+
+
 def test_decode_over_an_empty_request_table():
     """No request asks nothing of the table; one that does is refused before any launch."""
     lib = _lib.load()
