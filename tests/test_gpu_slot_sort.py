@@ -36,6 +36,38 @@ def test_gate_at_cluster_edges(cuda_device, S, E, k, cf):
     torch.testing.assert_close(w.cpu(), rw, rtol=1e-5, atol=1e-7)
 
 
+@pytest.mark.parametrize("S,E,k,capacity,blocks", [(1, 4, 1, 1, 1), (37, 8, 8, 5, 7), (4096, 64, 8, 640, 64), (3001, 512, 2, 3, 3001),
+                                                   (20000, 40, 4, 3000, 256)])
+def test_gate_then_assign_is_the_forward(cuda_device, S, E, k, capacity, blocks):
+    """The two-step C entries against the one the wrapper calls: the same choices, queues, lists and weights; the column
+    means are added in another order (fp32 sums of S values in [0, 1])."""
+    lib, stream = _lib.load(), _lib.stream_ptr(cuda_device)
+    x = torch.randn(S, E, generator=torch.Generator().manual_seed(S)).to(cuda_device)
+
+    def buffers():
+        new = lambda n, dt: torch.full((n,), -7, dtype=dt, device=cuda_device)      # noqa: E731
+        return [new(k * S, torch.int32), new(E, torch.float32), new(E, torch.float32), new(1, torch.float32),
+                new(k * S, torch.int32), new(k * S, torch.float32), new(E * capacity, torch.int64)]
+
+    gates, gates2 = torch.empty_like(x), torch.empty_like(x)
+    ids, ids_km = (torch.empty(S * k, dtype=torch.int32, device=cuda_device) for _ in range(2))
+    scratch = torch.empty(S * max(k, E), device=cuda_device)
+    one, two = buffers(), buffers()
+    _lib.check(lib.dlb_gshard_forward(x.data_ptr(), S, E, k, capacity, gates.data_ptr(), ids_km.data_ptr(),
+                                      scratch.data_ptr(), scratch.numel(), *[t.data_ptr() for t in one], stream), "forward")
+    _lib.check(lib.dlb_gshard_gate(x.data_ptr(), S, E, k, gates2.data_ptr(), ids.data_ptr(), scratch.data_ptr(), stream), "gate")
+    choices = ids.view(S, k).t().contiguous()
+    colsum = torch.empty(blocks * E, device=cuda_device)
+    _lib.check(lib.dlb_gshard_assign(gates2.data_ptr(), choices.data_ptr(), None, None, S, E, k, capacity,
+                                     colsum.data_ptr(), blocks, *[t.data_ptr() for t in two], stream), "assign")
+    assert torch.equal(gates, gates2) and torch.equal(ids_km, choices.view(-1))
+    for i, (a, b) in enumerate(zip(one, two)):
+        if i in (1, 3):      # me, l_aux
+            torch.testing.assert_close(a, b, rtol=1e-5, atol=0)
+        else:
+            assert torch.equal(a, b), i
+
+
 @pytest.mark.parametrize("E,k", [(8, 8), (5, 3), (40, 20)])
 def test_gate_of_a_negative_nan(cuda_device, E, k):
     """The fillers of a ragged gate rank above it: no id outside the experts, forward and backward (nothing reads or
