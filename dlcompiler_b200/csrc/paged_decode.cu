@@ -90,8 +90,7 @@ struct DecodeParams {
   int64_t o_stride_b, o_stride_h;
   int64_t bt_stride;
   const void* table_rows;    // [B] row of the block table of every sequence (int32 or int64), or null: row b
-  int num_table_rows, rows_is_int64;
-  int rows_gathered;         // the table holds the named rows in the order of the batch: row b, if the named one exists
+  int num_table_rows, rows_is_int64;   // + 2: the table holds the named rows in the order of the batch
   int batch, hq, hkv, group;
   int dk, dv;                // true head sizes of q/k and of v/out (<= D, multiples of 8); columns beyond them are zero
   int page_size, max_pages, num_pages;
@@ -131,8 +130,8 @@ __device__ __forceinline__ int load_index(const void* p, int64_t i, int is64) {
 
 // Row of the block table that sequence b reads, as it stands in table_rows (64 bits: not cut before it is compared).
 __device__ __forceinline__ int64_t named_row(const DecodeParams& p, int b) {
-  return p.rows_is_int64 ? reinterpret_cast<const int64_t*>(p.table_rows)[b]
-                         : reinterpret_cast<const int32_t*>(p.table_rows)[b];
+  return (p.rows_is_int64 & 1) ? reinterpret_cast<const int64_t*>(p.table_rows)[b]
+                               : reinterpret_cast<const int32_t*>(p.table_rows)[b];
 }
 
 // Token range [lo, hi) of split `s`; returns false if the split is empty.
@@ -146,9 +145,11 @@ __device__ __forceinline__ bool split_range(int ctx, int window, int chunk, int 
   return lo < hi;
 }
 
-// ROWS: the table's rows are found through table_rows (an instantiation of its own: the extra value made the plain one
-// 0.5 % slower on 64 sequences of 1k to 32k tokens).
-template <typename T, int D, bool ROWS>
+// How a sequence finds its row of the table.  An instantiation each: at 128 registers one more value costs a spill (the
+// named row made the plain form 0.5 % slower on 64 sequences of 1k to 32k tokens; a parameter that tells gathered from
+// named rows the named form 0.9 %, 216.1 -> 218.1 us for the token-granular decode of 16 sequences).
+enum { ROW_OWN, ROW_NAMED, ROW_GATHERED };
+template <typename T, int D, int ROWS>
 __global__ void __launch_bounds__(pd::THREADS + 32 * (pd::GATHER_WARPS - 1), 2)
 paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                           const DecodeParams p) {
@@ -176,7 +177,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
 
   int ctx = load_index(p.kv_seqlens, b, p.lens_is_int64);
   int64_t table_row = b;
-  if constexpr (ROWS) {
+  if constexpr (ROWS != ROW_OWN) {
     // a row outside the table names nobody's tokens: the sequence counts as empty and the call is recorded as wrong
     table_row = named_row(p, b);
     if (table_row < 0 || table_row >= p.num_table_rows) {
@@ -188,7 +189,7 @@ paged_decode_split_kernel(const __grid_constant__ CUtensorMap tmap_k, const __gr
         p.status[3] = (int)max((int64_t)INT32_MIN, min(table_row, (int64_t)INT32_MAX));
       }
     }
-    if (p.rows_gathered) table_row = b;
+    if constexpr (ROWS == ROW_GATHERED) table_row = b;
   }
   int lo, hi, kv_lo;
   if (!split_range(ctx, p.window, p.chunk, split, lo, hi, kv_lo)) {
@@ -578,7 +579,9 @@ static int launch_decode(const CUtensorMap& tk, const CUtensorMap& tv, const Dec
   constexpr int RED_BYTES = CONSUMER_WARPS * 16 * (D + 2) * 4;
   constexpr int RING = STAGES * STAGE_BYTES;
   constexpr int SMEM = (RING > RED_BYTES ? RING : RED_BYTES) + 1024 + 128;
-  auto kern = p.table_rows != nullptr ? paged_decode_split_kernel<T, D, true> : paged_decode_split_kernel<T, D, false>;
+  auto kern = p.table_rows == nullptr ? paged_decode_split_kernel<T, D, ROW_OWN>
+              : (p.rows_is_int64 & 2) ? paged_decode_split_kernel<T, D, ROW_GATHERED>
+                                      : paged_decode_split_kernel<T, D, ROW_NAMED>;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) {
     set_last_error("paged_decode: cannot raise dynamic shared memory: %s", cudaGetErrorString(e));
@@ -662,8 +665,7 @@ extern "C" int dlb_paged_decode_rows(const void* q, const void* k_cache, const v
   p.bt_stride = bt_stride;
   p.table_rows = table_rows;
   p.num_table_rows = (int)num_table_rows;
-  p.rows_is_int64 = rows_is_int64 & 1;
-  p.rows_gathered = rows_is_int64 & 2;
+  p.rows_is_int64 = rows_is_int64;
   p.batch = (int)batch;
   p.hq = (int)hq;
   p.hkv = (int)hkv;
