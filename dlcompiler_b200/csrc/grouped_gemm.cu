@@ -103,10 +103,10 @@ template <typename T> __device__ __forceinline__ float round_to(float a) { retur
 
 // x / (1 + e^-x), the quotient from an approximate reciprocal and one residual correction (Newton-Raphson on the
 // quotient, as in Markstein's division), without a branch.  An IEEE division per element, with its branch for the ends
-// of the range, kept the 32 elements of a step from overlapping: the epilogue of a tile took about 55 000 clocks, and
-// every gate/up launch with a shorter main loop waited for it (32 experts, K = 1024: 235 us for 369 MB of weights).
-// Whole fused_moe, before -> after: 2000 tokens over 256 experts (2048 x 1024) 676 -> 600 us, 128 over 64 (2048 x 1408)
-// 246 -> 203, 32 over 32 (1024 x 2816) 195 -> 113, 4096 over 8 (4096 x 14336) 2394 -> 2298.
+// of the range, keeps the 32 elements of a step from overlapping: the epilogue of a tile takes about 55 000 clocks, and
+// every gate/up launch with a shorter main loop waits for it.  Whole fused_moe with the division -> so (cold L2): 2000
+// tokens over 256 experts (top 8, 2048 x 1024) 692 -> 606 us, 128 over 64 (top 6, 2048 x 1408) 438 -> 225, 32 over 32
+// (top 4, 1024 x 2816) 313 -> 137, 4096 over 8 (top 2, 4096 x 14336) 2369 -> 2301.
 // Both sides are scaled by 1/4 so that the reciprocal of the largest 1 + e^-x is not subnormal.  Where e^-x is infinite
 // (x below -88.7) the quotient is -0, or NaN at -inf; at +inf the correction would make it NaN.  Rounded to the type,
 // every 16-bit x gives what the division gives.
@@ -531,9 +531,12 @@ static int grouped_gemm_impl(const void* a, int64_t a_rows, int64_t a_row_stride
 
   // Padding a third of the row list or more: few rows per block, the launch waits for the weights, and whole boxes of
   // A would add half of their bytes.  With full blocks the tensor cores' power is the limit and the few rows of padding
-  // had better be the zeros that moe_permute_slots makes them.
-  // Measured, whole fused_moe, before -> after: 32 tokens over 8 experts (4096 x 14336) 503 -> 477 us, 2000 over 256
-  // (2048 x 1024) 773 -> 687, 128 over 64 (2048 x 1408) 265 -> 248, 4096 over 32 (1024 x 2816) 575 -> 547.
+  // had better be the zeros that moe_permute_slots makes them.  The share is the worst case of the sizes, the counts
+  // being on the device: routing that fills a few of the experts alone takes the form that suits it less.
+  // Measured, whole fused_moe, cold L2, without -> with the form: 32 tokens over 8 experts (top 2, 4096 x 14336)
+  // 502 -> 474 us, 2000 over 256 (top 8, 2048 x 1024) 621 -> 606, 128 over 64 (top 6, 2048 x 1408) 234 -> 225, 4096 over
+  // 32 (top 2, 1024 x 2816) 217 -> 213; at the rule's line, 1000 over 8 (top 2, 4096 x 14336), 779 -> 769; 2000 tokens
+  // whose six choices are the same six or eight of 64 experts 248 -> 275 and 236 -> 267.
   const bool few = slots_only && (a_rows - numel) * 2 >= numel &&
                    (flags == FLAG_FUSE_SILU || flags == (FLAG_WEIGHT | FLAG_SCATTER));
 

@@ -21,7 +21,8 @@ constexpr int SORT_THREADS = 1024;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
 constexpr int SORT_MAX_CLUSTER = 8;     // the portable cluster size
 
-// CTAs for `numel` slots: a warp's segment stays at one to four rounds of 32 slots as long as eight CTAs allow.
+// CTAs for `numel` slots: a warp's segment is at most two rounds of 32 slots up to 16384 slots, with eight CTAs; it grows
+// with the slots after that.
 inline int sort_cluster_size(int64_t numel) {
   int c = 1;
   while (c < SORT_MAX_CLUSTER && numel > (int64_t)c * 2048) c <<= 1;
@@ -82,7 +83,7 @@ struct SlotSort {
   }
 
   // Fills count / before (all CTAs of the cluster take part).  The caller must keep the CTA alive until every
-  // other CTA has passed its own call: release() / finish().
+  // other CTA has passed its own call: finish().
   template <typename IdAt> __device__ __forceinline__ void count_slots(IdAt id_at) {
     int* mine = table + (threadIdx.x >> 5) * pitch;
     walk(id_at, [&](int, int e) {
