@@ -54,7 +54,8 @@ constexpr int KV_STAGES = 2;
 constexpr int TMEM_COLS = 256;    // S0 [0,64) S1 [64,128) O [128,128+D)
 constexpr float RESCALE_THRESHOLD = 8.0f;   // log2 units
 constexpr int64_t L2_BYTES = 126 << 20;
-enum { ORDER_GROUPS, ORDER_SORTED, ORDER_TILES, ORDER_RAGGED };
+enum { ORDER_GROUPS, ORDER_TILES, ORDER_RAGGED };                // of a packed launch
+enum { FORM_PACKED, FORM_PAGED, FORM_PAGED_SORTED };             // K/V packed or in pages; its order, see prefill_tile
 // (Computing a share of the exponentials with a degree-3 polynomial on the FMA pipe instead of the SFU,
 // as large kernels of this kind do, was measured on B200 at 12.5 %, 25 % and 37.5 % of the scores and
 // was 2 %, 4 % and 10 % slower on the 4 x 8192 benchmark: the softmax warps are bound by issue slots
@@ -140,7 +141,7 @@ struct PrefillParams {
   int batch, hq, hkv, group;
   int max_tiles;
   int causal;
-  int order;                      // of the CTAs, see prefill_tile
+  int order;                      // of a packed launch's CTAs, see prefill_tile
   float scale_log2;               // sm_scale * log2(e)
   uint32_t idesc_qk, idesc_pv;
   uint32_t v_lbo, v_sbo;          // MN-major descriptor strides of the V tile
@@ -148,7 +149,6 @@ struct PrefillParams {
   // Paged K/V (prefill over a cache that already holds kv_seq_len - seq_len earlier tokens of each
   // sequence): tmap_k / tmap_v are then 4-D maps over [pages, slots, heads, d] and the keys of a
   // sequence are found through its row of the block table.
-  int paged;
   int page_size, num_pages, max_pages;
   const void* block_table;        // [batch, max_pages] int32 or int64
   int64_t bt_stride;
@@ -176,7 +176,8 @@ __device__ __forceinline__ int table_entry(const void* t, int64_t i, int is64) {
 //   ORDER_GROUPS      (sequence, kv head) groups one after the other, inside a group the heavy (late, causal) tiles
 //                     first, the q heads of the group adjacent.  The CTAs resident at any time then share the K/V of one
 //                     or two groups (4 MiB each at 8k tokens), which stay in L2 instead of being re-read from HBM.
-//   ORDER_SORTED      the same with the sequences by descending key count: a long history must not start last.
+//                     Paged launches too (FORM_PAGED).
+//   FORM_PAGED_SORTED the same with the sequences by descending key count: a long history must not start last.
 //   ORDER_TILES       the row tile slowest, so that the heavy tiles of all groups come first and the launch ends on
 //                     light ones; for K/V that stay in L2 altogether.
 //   ORDER_RAGGED      ORDER_TILES over the tiles that exist, the CTAs without work last: on 13 prompts of 17 to 901
@@ -184,32 +185,52 @@ __device__ __forceinline__ int table_entry(const void* t, int64_t i, int is64) {
 // The sorted forms keep one sequence per lane (batch <= 32).  Measured on B200, 32 / 8 heads of 128, causal, cold L2, with
 // the early first loads and the epilogue below, ORDER_GROUPS for all with neither -> now: 1 x 2048 tokens 67.9 -> 55.1 us,
 // 1 x 8192 522 -> 472, 8 x 2048 346 -> 313, 64 x 256 135.0 -> 127.4, 64 x 64 46.8 -> 45.4, 13 prompts 88.8 -> 84.3.
-__device__ __forceinline__ bool prefill_tile(const PrefillParams& p, int x, int& seq, int& tile, int& head) {
-  if (p.order == fp::ORDER_GROUPS) {
+template <int FORM>
+__device__ __forceinline__ bool prefill_tile(const PrefillParams& p, int x, int& seq, int& tile, int& head, int& seq_len,
+                                             int& start, int& kv_len) {
+  auto fetch = [&] {
+    seq_len = p.b_seq_len[seq];
+    start = p.b_start_loc[seq];
+    kv_len = FORM != fp::FORM_PACKED ? p.kv_seq_len[seq] : seq_len;
+  };
+  if (FORM == fp::FORM_PAGED || (FORM == fp::FORM_PACKED && p.order == fp::ORDER_GROUPS)) {
     const int hig = x % p.group;
     x /= p.group;
     tile = p.max_tiles - 1 - x % p.max_tiles;
     x /= p.max_tiles;
     head = x % p.hkv * p.group + hig;
     seq = x / p.hkv;
+    fetch();
     return true;
   }
-  if (p.order == fp::ORDER_TILES) {
+  if (FORM == fp::FORM_PACKED && p.order == fp::ORDER_TILES) {
     head = x % p.hq;
     x /= p.hq;
     seq = x % p.batch;
     tile = p.max_tiles - 1 - x / p.batch;
+    fetch();
     return true;
   }
   const int lane = threadIdx.x & 31;
-  const int mine = lane < p.batch ? (p.paged ? p.kv_seq_len : p.b_seq_len)[lane] : -1;
-  int place = 0;                       // this lane's sequence among the lengths in descending order
-  for (int j = 0; j < p.batch; ++j) {
-    const int v = __shfl_sync(0xffffffffu, mine, j);
-    place += v > mine || (v == mine && j < lane) ? 1 : 0;
+  // one sequence per lane: all its sizes are fetched at once and handed out by shuffles
+  const bool has = lane < p.batch;
+  const int q_mine = has ? p.b_seq_len[lane] : 0, start_mine = has ? p.b_start_loc[lane] : 0;
+  const int mine = has ? (FORM != fp::FORM_PACKED ? p.kv_seq_len[lane] : q_mine) : -1;
+  // this lane's place among the lengths in descending order; chunks whose lengths differ by less than a quarter stay as
+  // they are, without the comparisons (32 x 64 tokens over 100, warm L2: 39.3 us with them, 37.3 without)
+  const int longest = __reduce_max_sync(0xffffffffu, mine);
+  const bool even = FORM == fp::FORM_PAGED_SORTED &&
+                    __reduce_min_sync(0xffffffffu, has ? mine : longest) >= longest - (longest >> 2);
+  int place = even ? lane : 0;
+  for (int j0 = 0; !even && j0 < p.batch; j0 += 8) {
+#pragma unroll
+    for (int j = j0; j < j0 + 8; ++j) {      // lanes without a sequence (-1) come after every other
+      const int v = __shfl_sync(0xffffffffu, mine, j);
+      place += v > mine || (v == mine && j < lane) ? 1 : 0;
+    }
   }
   int turn;
-  if (p.order == fp::ORDER_SORTED) {
+  if (FORM == fp::FORM_PAGED_SORTED) {
     const int hig = x % p.group;
     x /= p.group;
     tile = p.max_tiles - 1 - x % p.max_tiles;
@@ -230,28 +251,29 @@ __device__ __forceinline__ bool prefill_tile(const PrefillParams& p, int x, int&
     turn = x / p.hq;
     head = x - turn * p.hq;
   }
-  seq = __ffs(__ballot_sync(0xffffffffu, lane < p.batch && place == turn)) - 1;
+  seq = __ffs(__ballot_sync(0xffffffffu, has && place == turn)) - 1;
+  seq_len = __shfl_sync(0xffffffffu, q_mine, seq);
+  start = __shfl_sync(0xffffffffu, start_mine, seq);
+  kv_len = __shfl_sync(0xffffffffu, mine, seq);
   return true;
 }
 
-template <typename T, int D, bool EXTRAS>
+template <typename T, int D, bool EXTRAS, int FORM>
 __global__ void __launch_bounds__(fp::THREADS, 2)
 flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,
                      const __grid_constant__ CUtensorMap tmap_v, const PrefillParams p) {
   using namespace fp;
   using L = Layout<D>;
+  constexpr bool PAGED = FORM != FORM_PACKED;
   constexpr int BOXES = L::BOXES;
   constexpr int Q_BYTES = L::Q_BYTES, KV_BYTES = L::KV_BYTES;
   constexpr int OFF_Q = L::OFF_Q, OFF_K = L::OFF_K, OFF_V = L::OFF_V, OFF_CTRL = L::OFF_CTRL;
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   // ---- which tile ----
-  int seq, tile, head;
-  if (!prefill_tile(p, (int)blockIdx.x, seq, tile, head)) return;
+  int seq, tile, head, seq_len, start, kv_len;
+  if (!prefill_tile<FORM>(p, (int)blockIdx.x, seq, tile, head, seq_len, start, kv_len)) return;
   const int kvh = head / p.group;
-  const int seq_len = p.b_seq_len[seq];
-  const int start = p.b_start_loc[seq];
-  const int kv_len = p.paged ? p.kv_seq_len[seq] : seq_len;
   const int q0 = tile * BM;
   if (q0 >= seq_len) return;
   // query row r of the tile sits at position hist + q0 + r of its sequence (hist = tokens already cached)
@@ -286,7 +308,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   // of block j + 1 are fetched right after block j's K loads are issued, so that the look-up's latency never sits
   // between a freed stage and its next load.
   const int box_slots = min(p.page_size, BN);
-  const int n_sub = p.paged ? BN / box_slots : 0;
+  const int n_sub = PAGED ? BN / box_slots : 0;
   int pg[4] = {0, 0, 0, 0}, sl[4] = {0, 0, 0, 0};
   auto look_up = [&](int j) {
 #pragma unroll
@@ -305,7 +327,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                         const int (&slot)[4]) {
     uint8_t* dst = smem + off + (j & 1) * KV_BYTES;
     mbar_arrive_expect_tx(&full[j & 1], KV_BYTES);
-    if (p.paged) {
+    if constexpr (PAGED) {
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (u >= n_sub) break;
@@ -319,6 +341,11 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         tma_load_3d(dst + bx * KV_BOX, tmap, &full[j & 1], bx * 64, kvh, start + (jb0 + j) * BN);
     }
   };
+  auto load_q = [&] {
+    mbar_arrive_expect_tx(q_full, Q_BYTES);
+#pragma unroll
+    for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(smem + OFF_Q + bx * Q_BOX, &tmap_q, q_full, bx * 64, head, start + q0);
+  };
   if (warp == WARP_TMA && lane == 0) {
     mbar_init(q_full, 1);
     mbar_init(q_ready, 128);
@@ -331,15 +358,14 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
     *abort_flag = 0;
     fence_mbar_init();
-    // Q and the first K and V block are on their way while the rest of the CTA sets up
-    mbar_arrive_expect_tx(q_full, Q_BYTES);
-#pragma unroll
-    for (int bx = 0; bx < BOXES; ++bx) tma_load_3d(smem + OFF_Q + bx * Q_BOX, &tmap_q, q_full, bx * 64, head, start + q0);
-    if (nb > 0) {
-      look_up(0);
-      load_block(0, OFF_K, &tmap_k, k_full, pg, sl);
-      load_block(0, OFF_V, &tmap_v, v_full, pg, sl);
-      if (nb > 1) look_up(1);
+    if constexpr (!PAGED) {
+      // Q and the first K and V block are on their way while the rest of the CTA sets up.  With pages the look-up in front
+      // of them would hold up the whole CTA (64 chunks of 64 tokens over 100, warm L2: 62.8 us later, 64.0 here).
+      load_q();
+      if (nb > 0) {
+        load_block(0, OFF_K, &tmap_k, k_full, pg, sl);
+        load_block(0, OFF_V, &tmap_v, v_full, pg, sl);
+      }
     }
   }
   if (warp == WARP_MMA) {
@@ -354,7 +380,14 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
   if (warp == WARP_TMA) {
     if (lane == 0) {
-      for (int j = 1; j < nb; ++j) {
+      if constexpr (PAGED) {
+        tma_prefetch_desc(&tmap_q);
+        tma_prefetch_desc(&tmap_k);
+        tma_prefetch_desc(&tmap_v);
+        load_q();
+        if (nb > 0) look_up(0);
+      }
+      for (int j = PAGED ? 0 : 1; j < nb; ++j) {
         const int s = j & 1;
         const uint32_t ph = (j >> 1) & 1;
         int pv[4], sv[4];   // block j's pages for the V loads below
@@ -367,7 +400,7 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // (pv_done): no separate "empty" commits, every commit costs the single issuing thread ~100 clocks
         if (!mbar_wait(&s_full[s], ph ^ 1, abort_flag, p.status, 21, j)) break;
         load_block(j, OFF_K, &tmap_k, k_full, pg, sl);
-        if (j + 1 < nb) look_up(j + 1);
+        if (PAGED && j + 1 < nb) look_up(j + 1);
         if (!mbar_wait(&pv_done[s], ph ^ 1, abort_flag, p.status, 22, j)) break;
         load_block(j, OFF_V, &tmap_v, v_full, pv, sv);
       }
@@ -695,10 +728,10 @@ flash_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   }
 }
 
-template <typename T, int D, bool EXTRAS>
+template <typename T, int D, bool EXTRAS, int FORM>
 static int launch_prefill_x(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv,
                             const PrefillParams& p, unsigned grid, cudaStream_t stream) {
-  auto kern = flash_prefill_kernel<T, D, EXTRAS>;
+  auto kern = flash_prefill_kernel<T, D, EXTRAS, FORM>;
   constexpr int SMEM = fp::Layout<D>::SMEM_BYTES;
   cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
   if (e != cudaSuccess) {
@@ -708,11 +741,21 @@ static int launch_prefill_x(const CUtensorMap& tq, const CUtensorMap& tk, const 
   kern<<<grid, fp::THREADS, SMEM, stream>>>(tq, tk, tv, p);
   return DLB_OK;
 }
-template <typename T, int D>
+template <typename T, int D, int FORM>
 static int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p,
                           unsigned grid, cudaStream_t stream) {
-  return (p.window > 0 || p.softcap > 0.f) ? launch_prefill_x<T, D, true>(tq, tk, tv, p, grid, stream)
-                                           : launch_prefill_x<T, D, false>(tq, tk, tv, p, grid, stream);
+  if constexpr (FORM != fp::FORM_PACKED)
+    if (p.window > 0 || p.softcap > 0.f) return launch_prefill_x<T, D, true, FORM>(tq, tk, tv, p, grid, stream);
+  return launch_prefill_x<T, D, false, FORM>(tq, tk, tv, p, grid, stream);
+}
+template <int FORM>
+static int launch_prefill(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const PrefillParams& p, int D,
+                          int dtype, unsigned grid, cudaStream_t stream) {
+  if (dtype == DLB_DTYPE_BF16)
+    return D == 128 ? launch_prefill<__nv_bfloat16, 128, FORM>(tq, tk, tv, p, grid, stream)
+                    : launch_prefill<__nv_bfloat16, 64, FORM>(tq, tk, tv, p, grid, stream);
+  return D == 128 ? launch_prefill<__half, 128, FORM>(tq, tk, tv, p, grid, stream)
+                  : launch_prefill<__half, 64, FORM>(tq, tk, tv, p, grid, stream);
 }
 
 }  // namespace dlb
@@ -785,7 +828,6 @@ extern "C" int dlb_flash_prefill_varlen(const void* q, const void* k, const void
     const bool ragged = max_tiles * batch * 4 > (total_tokens / BM + batch) * 5;
     p.order = !ragged ? ORDER_TILES : batch <= 32 ? ORDER_RAGGED : ORDER_GROUPS;
   }
-  p.paged = 0;
   p.page_size = BN;
   p.num_pages = p.max_pages = 0;
   p.block_table = nullptr;
@@ -804,14 +846,7 @@ extern "C" int dlb_flash_prefill_varlen(const void* q, const void* k, const void
   p.sm_scale = sm_scale;
 
   cudaStream_t s = (cudaStream_t)stream;
-  int rc2;
-  if (dtype == DLB_DTYPE_BF16) {
-    rc2 = D == 128 ? launch_prefill<__nv_bfloat16, 128>(tq, tk, tv, p, (unsigned)grid, s)
-                   : launch_prefill<__nv_bfloat16, 64>(tq, tk, tv, p, (unsigned)grid, s);
-  } else {
-    rc2 = D == 128 ? launch_prefill<__half, 128>(tq, tk, tv, p, (unsigned)grid, s)
-                   : launch_prefill<__half, 64>(tq, tk, tv, p, (unsigned)grid, s);
-  }
+  const int rc2 = launch_prefill<FORM_PACKED>(tq, tk, tv, p, D, dtype, (unsigned)grid, s);
   if (rc2 != DLB_OK) return rc2;
   DLB_CUDA_LAUNCH_CHECK();
   return DLB_OK;
@@ -888,9 +923,7 @@ extern "C" int dlb_flash_prefill_paged(const void* q, const void* k_cache, const
   p.v_lbo = KV_BOX;
   p.v_sbo = 1024;
   p.status = status;
-  // a launch that starts all its CTAs at once gains nothing from their order
-  p.order = batch > 1 && batch <= 32 && grid > 2 * sm_count(current_device()) ? ORDER_SORTED : ORDER_GROUPS;
-  p.paged = 1;
+  p.order = ORDER_GROUPS;
   p.page_size = (int)page_size;
   p.num_pages = (int)num_pages;
   p.max_pages = (int)max_pages;
@@ -912,14 +945,13 @@ extern "C" int dlb_flash_prefill_paged(const void* q, const void* k_cache, const
   p.sm_scale = sm_scale;
 
   cudaStream_t s = (cudaStream_t)stream;
-  int rc2;
-  if (dtype == DLB_DTYPE_BF16) {
-    rc2 = D == 128 ? launch_prefill<__nv_bfloat16, 128>(tq, tk, tv, p, (unsigned)grid, s)
-                   : launch_prefill<__nv_bfloat16, 64>(tq, tk, tv, p, (unsigned)grid, s);
-  } else {
-    rc2 = D == 128 ? launch_prefill<__half, 128>(tq, tk, tv, p, (unsigned)grid, s)
-                   : launch_prefill<__half, 64>(tq, tk, tv, p, (unsigned)grid, s);
-  }
+  // A launch that starts all its CTAs at once gains nothing from their order, and where the table has no room for 512 keys
+  // more than the new tokens no history can be long.  16 chunks of 64 tokens over 100 or 4000 in turn, warm L2: 130 us in
+  // the order of the batch, 80 sorted; 8 of 512 over 2000 each, which it cannot help: 171 and 172.
+  const bool sorted = batch > 1 && batch <= 32 && grid > 2 * sm_count(current_device()) &&
+                      max_pages * page_size > max_q_len + 512;
+  const int rc2 = sorted ? launch_prefill<FORM_PAGED_SORTED>(tq, tk, tv, p, D, dtype, (unsigned)grid, s)
+                         : launch_prefill<FORM_PAGED>(tq, tk, tv, p, D, dtype, (unsigned)grid, s);
   if (rc2 != DLB_OK) return rc2;
   DLB_CUDA_LAUNCH_CHECK();
   return DLB_OK;

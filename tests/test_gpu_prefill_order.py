@@ -51,13 +51,12 @@ def test_epilogue_by_rows_of_the_tile(cuda_device, rows, dim):
     assert (wide[rows:] == 7).all() and (wide[:, :, dim:] == 7).all()
 
 
-@pytest.mark.parametrize("batch", [5, 32, 33])
-def test_paged_sequences_by_length(cuda_device, batch):
-    """More tiles than the GPU holds at once: sequences by descending key count, up to 32 of them.  A sequence
-    attends to its own keys only, so every one must equal a launch of its own (which starts all tiles at once)."""
+def _each_as_if_alone(cuda_device, batch, history):
+    """A sequence attends to its own keys only, so every one must equal a launch of its own (which starts all tiles at
+    once)."""
     hq, hkv, dim, page = 32, 8, 64, 16
     lens = [150 if i % 3 else 40 for i in range(batch)]
-    full = [n + (37 * i) % 200 for i, n in enumerate(lens)]
+    full = [n + history(i) for i, n in enumerate(lens)]
     q, _, _, start, n = _case(lens, hq, hkv, dim, batch)
     g = torch.Generator().manual_seed(1)
     pages = [(m + page - 1) // page for m in full]
@@ -75,3 +74,18 @@ def test_paged_sequences_by_length(cuda_device, batch):
         paged_attention_fwd(q[rows], kc, vc, alone, table[b:b + 1], torch.zeros(1, dtype=torch.int32, device=cuda_device),
                             n[b:b + 1].to(cuda_device), kv[b:b + 1], lens[b])
         assert torch.equal(o[rows], alone)
+
+
+@pytest.mark.parametrize("batch", [5, 32, 33])
+def test_paged_sequences_by_length(cuda_device, batch):
+    """More tiles than the GPU holds at once, in the order of the batch (short histories)."""
+    _each_as_if_alone(cuda_device, batch, lambda i: (37 * i) % 200)
+
+
+@pytest.mark.parametrize("batch", [5, 31, 32, 33])
+@pytest.mark.parametrize("history", ["about the same", "far apart", "equal pairs"])
+def test_paged_long_histories(cuda_device, batch, history):
+    """A table with room for long histories: up to 32 sequences by descending key count, or as they are when their lengths
+    are within a quarter."""
+    _each_as_if_alone(cuda_device, batch, {"about the same": lambda i: 900 + i, "far apart": lambda i: (397 * i) % 1700,
+                                           "equal pairs": lambda i: 1200 * (i // 2 % 2)}[history])
