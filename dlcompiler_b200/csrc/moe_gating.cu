@@ -530,10 +530,11 @@ static int launch_gating(const GatingParams& p_in, void* stream) {
 //   gates = softmax(logits); the k choices of every token queue up per expert in
 //   (choice-major, token) order; a choice is kept if its queue position is below the
 //   capacity; weights = kept gate values normalised over the token's kept choices.
-// Queue positions come from the stable counting sort of moe_align (block 1) over the
-// choice-major id list, so no [k, S, E] mask tensors are materialised.
+// Queue positions come from the stable slot sort (slot_sort.cuh) over the choice-major
+// id list, so no [k, S, E] mask tensors are materialised.
 // ----------------------------------------------------------------------------
-// Deterministic column sums of gates [S, E]: stage 1 reduces row chunks, stage 2 the partials.
+// Deterministic column sums of gates [S, E] over row chunks, for dlb_gshard_assign (dlb_gshard_forward has them from the
+// gate kernel); gshard_assign_kernel adds the partial sums.
 __global__ void __launch_bounds__(256) gshard_colsum_stage1(const float* __restrict__ gates, float* __restrict__ part,
                                                             int64_t S, int E, int rows_per_block) {
   const int64_t r0 = (int64_t)blockIdx.x * rows_per_block;

@@ -34,7 +34,7 @@ def test_rows_and_widths(cuda_device, rows, hidden, inter, dtype):
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_silu_over_its_range(cuda_device, dtype):
-    """The activation from one end of its range to the other: hidden state 1, gate weights the values, up weights 1 and
+    """The activation from -6e4 to 6e4 through the whole block: hidden state 1, gate weights the values, up weights 1 and
     an identity behind it give silu(value).  Two roundings to the type; below 2^-24 only the size is left to compare."""
     values = torch.cat([torch.linspace(-104, 104, 833), torch.tensor([-6e4, -500., -88.8, -87.4, 0., 1e-4, 500., 6e4])])
     n = values.numel() // 8 * 8
